@@ -505,6 +505,41 @@ int gmres_run(Handle* h, const double* d_b, double* x, double tol, int maxit, in
 
 int check_cs_fault(Handle* h);
 
+// The cooperative solve (pm_coop.cu) after the solver's init kernel.  A refused
+// launch, or a wait that gave up, leaves the solve to the phase kernels (which
+// start again from the init in the latter case), then and from now on.
+enum class Coop { kNotRun, kSolved, kGaveUp };
+int run_coop(Handle* h, bool sqmr, pm::KrylovScalars* ks, Coop* how) {
+  *how = Coop::kNotRun;
+  if (h->coop_failed || !pm::coop_fits(h->P.view(), h->P.nnz, h->sms) ||
+      std::getenv("PM_POLLED_GRAPHS"))
+    return PM_OK;
+  if (!h->D.coop) {
+    if (cudaMalloc(&h->D.coop, pm::coop_scratch_bytes()) != cudaSuccess) {
+      cudaGetLastError();
+      h->coop_failed = true;
+      return PM_OK;
+    }
+    PM_CUDA(cudaMemsetAsync(h->D.coop, 0, pm::coop_scratch_bytes(), h->stream));
+  }
+  if (pm::krylov_coop(sqmr, h->P.view(), h->P.val, h->D.m, h->D.kv, h->D.ks, h->D.coop,
+                      h->coop_epoch, h->sms, h->stream) != cudaSuccess) {
+    cudaGetLastError();  // the refusal is not this solve's error
+    h->coop_failed = true;
+    return PM_OK;
+  }
+  h->launches += 1;
+  PM_TRY(read_scalars(h, ks));
+  const bool done = ks->fault == 0 && ks->conv_flag != 0;
+  h->coop_epoch += (unsigned long long)pm::kCoopEpochs * (ks->iter + 1);
+  *how = done ? Coop::kSolved : Coop::kGaveUp;
+  if (!done) {
+    h->coop_failed = true;
+    if (h->debug) fprintf(stderr, "cooperative solve gave up: phase kernels\n");
+  }
+  return PM_OK;
+}
+
 // One Krylov solve of K x = b on the device (solv_pm, Solv.f:27-780).
 //
 // comp = false: the reference's FP64 iteration on the FP64 panels.
@@ -533,7 +568,23 @@ int krylov(Handle* h, int solver, const double* d_b, double* d_x, double tol, in
   PM_CUDA(cudaEventRecord(e0, h->stream));
   if (solver == 1) {
     cudaGraphExec_t* g = comp ? &h->pcgc_graph : &h->pcg_graph;
-    if (!*g) {
+    auto init = [&]() -> int {
+      h->launches += 1;
+      if (comp)
+        PM_CUDA(pm::pcgc_init(n, d_b, h->D.m, V, V32, h->D.ks, tol, -1.0, maxit, h->D.partial,
+                              h->D.counter, h->stream));
+      else
+        PM_CUDA(pm::pcg_init(n, d_b, h->D.m, V, h->D.ks, tol, maxit, h->D.partial, h->D.counter,
+                             h->stream));
+      return PM_OK;
+    };
+    PM_TRY(init());
+    Coop coop = Coop::kNotRun;
+    if (!comp) {
+      PM_TRY(run_coop(h, false, &ks, &coop));
+      if (coop == Coop::kGaveUp) PM_TRY(init());
+    }
+    if (coop != Coop::kSolved && !*g) {
       PM_TRY(capture(h, g, [&]() {
         return comp ? pm::pcgc_iteration(P, C, n, h->D.m, V, V32, h->D.ks, h->D.partial,
                                          h->D.counter, h->stream)
@@ -541,14 +592,9 @@ int krylov(Handle* h, int solver, const double* d_b, double* d_x, double tol, in
                                         h->D.counter, h->stream);
       }));
     }
-    h->launches += 1;
-    if (comp)
-      PM_CUDA(pm::pcgc_init(n, d_b, h->D.m, V, V32, h->D.ks, tol, -1.0, maxit, h->D.partial,
-                            h->D.counter, h->stream));
-    else
-      PM_CUDA(pm::pcg_init(n, d_b, h->D.m, V, h->D.ks, tol, maxit, h->D.partial, h->D.counter,
-                           h->stream));
-    if (!comp) {
+    if (coop == Coop::kSolved) {
+      // *ks holds the solve's flags
+    } else if (!comp) {
       PM_TRY(build_pcg_loop(h));
       if (h->pcg_loop) {
         PM_CUDA(cudaGraphLaunch(h->pcg_loop, h->stream));
@@ -759,15 +805,15 @@ int krylov(Handle* h, int solver, const double* d_b, double* d_x, double tol, in
     ks.iter = nit;
   } else if (solver == 11) {
     cudaGraphExec_t* g = comp ? &h->sqmrc_graph : &h->sqmr_graph;
-    if (!*g) {
-      PM_TRY(capture(h, g, [&]() {
-        return comp ? pm::sqmrc_iteration(P, C, n, h->D.m, V, V32, h->D.ks, h->D.partial,
-                                          h->D.counter, h->stream)
-                    : pm::sqmr_iteration(P, val64, n, h->D.m, V, h->D.ks, h->D.partial,
-                                         h->D.counter, h->stream);
-      }));
-    }
     auto run_sqmr = [&]() -> int {
+      if (!*g) {
+        PM_TRY(capture(h, g, [&]() {
+          return comp ? pm::sqmrc_iteration(P, C, n, h->D.m, V, V32, h->D.ks, h->D.partial,
+                                            h->D.counter, h->stream)
+                      : pm::sqmr_iteration(P, val64, n, h->D.m, V, h->D.ks, h->D.partial,
+                                           h->D.counter, h->stream);
+        }));
+      }
       for (;;) {
         PM_CUDA(cudaGraphLaunch(*g, h->stream));
         h->launches += 4 * kGraphIters;
@@ -775,10 +821,19 @@ int krylov(Handle* h, int solver, const double* d_b, double* d_x, double tol, in
         if (ks.conv_flag) return PM_OK;
       }
     };
-    h->launches += 1;
-    PM_CUDA(pm::sqmr_init(n, d_b, h->D.m, V, comp ? V32.c : nullptr, h->D.ks, tol, -1.0, maxit,
-                          h->D.partial, h->D.counter, h->stream));
-    PM_TRY(run_sqmr());
+    auto init = [&]() -> int {
+      h->launches += 1;
+      PM_CUDA(pm::sqmr_init(n, d_b, h->D.m, V, comp ? V32.c : nullptr, h->D.ks, tol, -1.0, maxit,
+                            h->D.partial, h->D.counter, h->stream));
+      return PM_OK;
+    };
+    PM_TRY(init());
+    Coop coop = Coop::kNotRun;
+    if (!comp) {
+      PM_TRY(run_coop(h, true, &ks, &coop));
+      if (coop == Coop::kGaveUp) PM_TRY(init());
+    }
+    if (coop != Coop::kSolved) PM_TRY(run_sqmr());
     int total = ks.iter;
     const double conv = ks.conv;
     // compensated operator: the FP64 residual b - A64 x (rpsqmr's 2-norm
@@ -1389,6 +1444,7 @@ void free_all(Handle* h) {
   if (h->pcg_graph) cudaGraphExecDestroy(h->pcg_graph);
   if (h->pcg_loop) cudaGraphExecDestroy(h->pcg_loop);
   if (h->D.trips) cudaFree(h->D.trips);
+  if (h->D.coop) cudaFree(h->D.coop);
   if (h->pcgm_graph) cudaGraphExecDestroy(h->pcgm_graph);
   if (h->minres_graph) cudaGraphExecDestroy(h->minres_graph);
   if (h->pcgc_graph) cudaGraphExecDestroy(h->pcgc_graph);
@@ -1973,6 +2029,10 @@ static int mesh_create(int nnode, int nnodev, int numel, int nen, int nenv, int 
   if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess)
     return fail(PM_E_CUDA);
   if (pm::ensure_shape_tables() != cudaSuccess) return fail(PM_E_CUDA);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return fail(PM_E_CUDA);
   for (auto& ev : h->ev)
     if (cudaEventCreate(&ev) != cudaSuccess) return fail(PM_E_CUDA);
   if ((st = pm::build_structure(h, ix, id, fnno, x, num)) != PM_OK) return fail(st);

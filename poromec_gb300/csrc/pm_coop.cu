@@ -1,0 +1,597 @@
+// pm_coop.cu -- a whole FP64 PCG or rpsqmr solve as one cooperative kernel.
+//
+// What bounds it.  With one kernel per phase an iteration of a small system is
+// launches, gaps and last-block reductions: 24.6 us for the 2,702 equations of
+// the 2 x 2 x 40 column, whose 273 k panel values take the FP64 pipe 0.5 us.
+// Here one CTA per SM stays on for the whole solve.  A CTA owns a set of nodes:
+// it multiplies their rows and keeps their entries of x, r, p, m and q in
+// shared memory, so only the direction p, gathered by all, goes through L2.
+// An iteration has three exchanges between the CTAs: (p, q), (r, z), and the
+// new direction's visibility.  The last one is saved where the panels have few
+// columns (FUSE): each gather then forms p = z + beta p_old itself, one more
+// FP64 instruction per column.
+//
+// Exchanges.  Every CTA stores its partial sum with an epoch, 16 bytes, into
+// its slot of kReplicas arrays; one warp of each CTA polls one array, all its
+// slots in flight together, and adds them in sender order.  The sum is the
+// same in every CTA, so all take the same decisions, and it does not depend on
+// the order of arrival.  Clocks of an exchange of 152 CTAs: 3,530 with 32
+// arrays, 3,780 with one per CTA, 4,070 with 8, 7,470 with one for all (its
+// readers queue at the same L2 slices); 1,470 of them are the FP64 adds.
+//
+// FP64 instructions set the rest: a dependent add takes 66 clocks and occupies
+// the scheduler's pipe for 64 whatever its mask, a division 1,430.  So the
+// reductions and the scalar recurrences run in one warp, the quotients come from
+// a Newton iteration (alpha) or a reciprocal formed ahead (beta), and the results
+// are broadcast.  The panels are read through L1, which holds them from one
+// iteration to the next where they fit.
+//
+// The recurrences and tests are those of the kernels in pm_sparse.cu
+// (k_pcg_update, k_sqmr_r, k_sqmr_x; Iters.f:299-595 and 6100-6439).  Every
+// wait is bounded: a CTA that gives up sets ks->fault and leaves, the others then
+// give up as well, and the host solves again with the phase kernels.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "pm_krylov.h"
+#include "pm_reduce.h"
+
+namespace pm {
+namespace {
+
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kCoopThreads = 512;
+constexpr int kCoopWarps = kCoopThreads / 32;
+constexpr int kCoopMaxCtas = 160;            // senders and receivers of an exchange
+constexpr int kReplicas = 32;                // arrays of slots (at most one per lane)
+constexpr int kPollLimit = 1 << 22;          // about 2 s of polling
+// columns per lane whose loads are in flight
+constexpr int chunk_of(bool fuse) { return fuse ? 5 : 9; }
+
+struct alignas(16) Slot {
+  double v;
+  unsigned long long epoch;
+};
+
+__device__ __forceinline__ void slot_store(Slot* s, double v, unsigned long long epoch) {
+  asm volatile(
+      "{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(s),
+      "l"(__double_as_longlong(v)), "l"(epoch)
+      : "memory");
+}
+__device__ __forceinline__ void slot_load(const Slot* s, double& v, unsigned long long& epoch) {
+  long long b;
+  asm volatile(
+      "{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+      : "=l"(b), "=l"(epoch)
+      : "l"(s)
+      : "memory");
+  v = __longlong_as_double(b);
+}
+
+struct CoopArgs {
+  int nloc;             // nodes per CTA (rounded up)
+  const double* m;
+  double *x, *r, *p;
+  double *p2, *z;       // FUSE: the other direction buffer, and z for the gathers
+  KrylovScalars* ks;
+  Slot* slots;
+  unsigned long long epoch;  // the slots' last epoch
+};
+
+// The CTA's shared memory: the nodes it owns and their entries, four per node.
+struct CoopShared {
+  double part[2][kCoopThreads];
+  double scal[8];
+  int flag, stop;
+};
+struct CoopLocal {
+  double *x, *r, *p, *m, *q, *d;
+  int64_t* vo;
+  int64_t* co;
+  int* e0;
+  int* dw;   // d | W << 3
+  int rows;  // 4 x nodes of this CTA
+};
+__host__ __device__ constexpr int coop_local_bytes(bool sqmr, int nloc) {
+  return nloc * (4 * (sqmr ? 6 : 5) * (int)sizeof(double) + 2 * (int)sizeof(int64_t) +
+                 2 * (int)sizeof(int));
+}
+
+// Group i of 32 / L nodes belongs to CTA i % G, whose warps take its groups in
+// turn, so all schedulers get equal shares of the sorted visiting order.
+template <int L>
+__device__ CoopLocal coop_setup(const PanelView& P, const CoopArgs& A, bool sqmr, double* dyn) {
+  constexpr int NPW = 32 / L;
+  CoopLocal S;
+  const size_t n4 = 4 * (size_t)A.nloc;
+  S.x = dyn;
+  S.r = S.x + n4;
+  S.p = S.r + n4;
+  S.m = S.p + n4;
+  S.q = S.m + n4;
+  S.d = S.q + n4;  // rpsqmr only
+  S.vo = reinterpret_cast<int64_t*>(sqmr ? S.d + n4 : S.d);
+  S.co = S.vo + A.nloc;
+  S.e0 = reinterpret_cast<int*>(S.co + A.nloc);
+  S.dw = S.e0 + A.nloc;
+  const int groups = (P.nact + NPW - 1) / NPW;
+  const int mine = (groups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  S.rows = 4 * NPW * mine;
+  for (int k = threadIdx.x; k < NPW * mine; k += kCoopThreads) {
+    const int slot = ((int)blockIdx.x + (k / NPW) * (int)gridDim.x) * NPW + k % NPW;
+    const NodeRef nr = node_ref(P, slot);
+    S.vo[k] = nr.vo;
+    S.co[k] = nr.co;
+    S.e0[k] = nr.e0;
+    S.dw[k] = nr.d | (nr.W << 3);
+    for (int j = 0; j < 4; ++j) {
+      const bool on = j < nr.d;
+      S.x[4 * k + j] = 0.0;
+      S.r[4 * k + j] = on ? A.r[nr.e0 + j] : 0.0;
+      S.p[4 * k + j] = on ? A.p[nr.e0 + j] : 0.0;
+      S.m[4 * k + j] = on ? A.m[nr.e0 + j] : 0.0;
+      S.q[4 * k + j] = 0.0;
+      if (sqmr) S.d[4 * k + j] = 0.0;
+    }
+  }
+  return S;
+}
+
+// q = A p on the CTA's nodes, L lanes per node; p (FUSE: z + beta p) is read
+// from L2 (other CTAs wrote it).  A lane's loads are issued chunk_of(FUSE)
+// columns at a time.
+template <int D, int L, bool FUSE>
+__device__ __forceinline__ void coop_rows(const double* __restrict__ v,
+                                          const int32_t* __restrict__ cols, const double* p,
+                                          const double* z, double beta, int W, int t,
+                                          double (&a)[4]) {
+  constexpr int kChunk = chunk_of(FUSE);
+  for (int c0 = 0; c0 < W; c0 += kChunk * L) {
+    double xv[kChunk], zv[FUSE ? kChunk : 1];
+    // columns past the last one repeat it and count zero: no branch holds back
+    // a load
+#pragma unroll
+    for (int u = 0; u < kChunk; ++u) {
+      const int c = cols[min(c0 + u * L + t, W - 1)];
+      xv[u] = __ldcg(&p[c]);
+      if (FUSE) zv[u] = __ldcg(&z[c]);
+    }
+#pragma unroll
+    for (int u = 0; u < kChunk; ++u) {
+      if (c0 + u * L >= W) break;
+      const int c = c0 + u * L + t;
+      const bool on = c < W;
+      if (FUSE) xv[u] = zv[u] + beta * xv[u];
+      const double x = on ? xv[u] : 0.0;
+      const double* vc = v + (on ? c : W - 1);
+#pragma unroll
+      for (int r = 0; r < D; ++r) a[r] += (on ? vc[r * W] : 0.0) * x;
+    }
+  }
+}
+
+template <int L, bool FUSE>
+__device__ void coop_spmv(const CoopLocal& S, const double* __restrict__ val,
+                          const int32_t* __restrict__ cols, const double* p, const double* z,
+                          double beta) {
+  constexpr int NPW = 32 / L;
+  const int lane = threadIdx.x & 31, t = lane & (L - 1);
+  for (int g = threadIdx.x >> 5; g < S.rows / (4 * NPW); g += kCoopWarps) {
+    const int k = g * NPW + lane / L;
+    const int d = S.dw[k] & 7, W = S.dw[k] >> 3;
+    const double* v = val + S.vo[k];
+    const int32_t* cl = cols + S.co[k];
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    if (d == 4) coop_rows<4, L, FUSE>(v, cl, p, z, beta, W, t, a);
+    else if (d == 3) coop_rows<3, L, FUSE>(v, cl, p, z, beta, W, t, a);
+    else if (d == 2) coop_rows<2, L, FUSE>(v, cl, p, z, beta, W, t, a);
+    else if (d == 1) coop_rows<1, L, FUSE>(v, cl, p, z, beta, W, t, a);
+    // transposed butterfly over the L lanes (k_spmv)
+    constexpr int o1 = L / 2, o2 = L / 4;
+    const bool h1 = (t & o1) != 0, h2 = (t & o2) != 0;
+    double k0 = h1 ? a[2] : a[0], k1 = h1 ? a[3] : a[1];
+    k0 += __shfl_xor_sync(kFull, h1 ? a[0] : a[2], o1);
+    k1 += __shfl_xor_sync(kFull, h1 ? a[1] : a[3], o1);
+    double kk = h2 ? k1 : k0;
+    kk += __shfl_xor_sync(kFull, h2 ? k0 : k1, o2);
+#pragma unroll
+    for (int o = L / 8; o > 0; o >>= 1) kk += __shfl_xor_sync(kFull, kk, o);
+    const int r = (h1 ? 2 : 0) + (h2 ? 1 : 0);
+    if ((t & (o2 - 1)) == 0 && r < d) S.q[4 * k + r] = kk;
+  }
+}
+
+// 1 / a by Newton's iteration x <- x + x (1 - a x) from the hardware's
+// approximation (20 bits: two steps); the division where that could leave the
+// normal range.
+__device__ __forceinline__ double recip(double a) {
+  const int e = (__double2hiint(a) >> 20) & 0x7ff;
+  if (e < 100 || e > 1946) return 1.0 / a;
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
+  x = fma(x, fma(-a, x, 1.0), x);
+  return fma(x, fma(-a, x, 1.0), x);
+}
+// b / a with one correction of the quotient's remainder
+__device__ __forceinline__ double quotient(double b, double a) {
+  const int e = (__double2hiint(b) >> 20) & 0x7ff;
+  const double x = recip(a);
+  if (e < 200 || e > 1846 || !isfinite(x)) return b / a;
+  const double q = b * x;
+  return fma(fma(-a, q, b), x, q);
+}
+
+// One exchange.  part[k][i], i < min(rows, kCoopThreads), are the CTA's terms of
+// value k; VIS (and NV = 0) makes the writes before it visible to all CTAs after
+// it.
+// Warp 0 sums, sends, polls, and has the NV totals in all its lanes; the other
+// warps return at once.  The caller broadcasts what follows from the totals.
+template <int NV, bool VIS = NV == 0>
+__device__ __forceinline__ bool exchange(CoopShared& S, const CoopArgs& A, int rows,
+                                         unsigned long long epoch, double (&tot)[NV > 0 ? NV : 1]) {
+  constexpr int N1 = NV > 0 ? NV : 1;
+  __syncthreads();
+  if (threadIdx.x >= 32) return true;
+  const int lane = threadIdx.x, G = gridDim.x;
+  double mine[N1] = {};
+  if (NV > 0) {
+    const int n = min(rows, kCoopThreads);
+#pragma unroll
+    for (int k = 0; k < N1; ++k) {
+      for (int i = lane; i < n; i += 32) mine[k] += S.part[k][i];
+      mine[k] = warp_sum(mine[k]);
+    }
+  }
+  if (VIS) __threadfence();
+  Slot* buf = A.slots + (size_t)(epoch & 1) * N1 * kReplicas * kCoopMaxCtas;
+  if (lane < kReplicas)
+#pragma unroll
+    for (int k = 0; k < N1; ++k)
+      slot_store(buf + ((size_t)lane * N1 + k) * kCoopMaxCtas + blockIdx.x, mine[k], epoch);
+  const Slot* in = buf + (size_t)(blockIdx.x % kReplicas) * N1 * kCoopMaxCtas;
+  double sum[N1] = {};
+  constexpr int kPer = kCoopMaxCtas / 32;
+  double got[N1][kPer];
+  // all of a lane's slots in flight together: an exchange then costs one or two
+  // load latencies, not one per slot
+  bool late = true;
+  for (int n = 0; n < kPollLimit && late; ++n) {
+    unsigned long long e[N1][kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+#pragma unroll
+      for (int k = 0; k < N1; ++k) {
+        got[k][j] = 0.0;
+        e[k][j] = epoch;
+        if (lane + 32 * j < G)
+          slot_load(in + (size_t)k * kCoopMaxCtas + lane + 32 * j, got[k][j], e[k][j]);
+      }
+    late = false;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+#pragma unroll
+      for (int k = 0; k < N1; ++k) late |= e[k][j] != epoch;
+  }
+  if (__any_sync(kFull, late)) return false;
+  if (VIS) __threadfence();
+  if (NV > 0) {
+#pragma unroll
+    for (int k = 0; k < N1; ++k) {
+#pragma unroll
+      for (int j = 0; j < kPer; ++j)
+        if (32 * j < G) sum[k] += got[k][j];
+      tot[k] = warp_sum(sum[k]);
+    }
+  }
+  return true;
+}
+
+// Terms of a dot product over the CTA's rows: term(i) for row i, one partial
+// per thread.
+template <typename F>
+__device__ __forceinline__ void coop_terms(double* part, int rows, F term) {
+  if ((int)threadIdx.x < rows) {
+    double acc = 0.0;
+    for (int i = threadIdx.x; i < rows; i += kCoopThreads) acc += term(i);
+    part[threadIdx.x] = acc;
+  }
+}
+
+#define COOP_SYNC()     \
+  do {                  \
+    __syncthreads();    \
+    if (S.stop) return; \
+  } while (0)
+
+// PCG: r = b, p = z = M r, d = (r, z) are k_pcg_init's.  Warp 0 keeps the
+// scalars.
+template <int L, bool FUSE>
+__global__ void __launch_bounds__(kCoopThreads, 1)
+    k_pcg_coop(PanelView P, const double* __restrict__ val, CoopArgs A) {
+  extern __shared__ double coop_dyn[];
+  __shared__ CoopShared S;
+  const CoopLocal X = coop_setup<L>(P, A, false, coop_dyn);
+  KrylovScalars* ks = A.ks;
+  const double conv = ks->conv;
+  const int maxit = ks->maxit;
+  // |d| at or above this is not converged whatever the rounding of the root
+  const double far = conv * conv * (1.0 + 1e-9);
+  double d = ks->d, rd = 1.0 / d;
+  unsigned long long epoch = A.epoch;
+  int iter = 0;
+  double pq = 0.0, beta = 0.0, alpha = 0.0;
+  double *pn = A.p, *po = A.p2;  // FUSE: the direction's buffers, newest first
+  if (threadIdx.x == 0) S.stop = 0;
+  __syncthreads();
+  coop_spmv<L, false>(X, val, P.cols, A.p, nullptr, 0.0);
+  for (;;) {
+    __syncthreads();
+    coop_terms(S.part[0], X.rows, [&](int i) { return X.p[i] * X.q[i]; });
+    double tot[1];
+    bool ok = exchange<1>(S, A, X.rows, ++epoch, tot);
+    if (threadIdx.x < 32) {
+      pq = tot[0];
+      alpha = quotient(d, pq);
+      if (threadIdx.x == 0) {
+        S.scal[0] = alpha;
+        S.flag = isfinite(alpha) ? 0 : 3;  // (p, A p) = 0: x stays as it is
+        if (!ok) S.stop = ks->fault = 1;
+      }
+    }
+    COOP_SYNC();
+    if (S.flag) break;
+    const double al = S.scal[0];
+    coop_terms(S.part[0], X.rows, [&](int i) {
+      X.x[i] = X.x[i] + al * X.p[i];
+      const double ri = X.r[i] - al * X.q[i];
+      X.r[i] = ri;
+      const double zi = ri * X.m[i];
+      X.q[i] = zi;  // q is done with: z
+      if (FUSE && (i & 3) < (X.dw[i >> 2] & 7)) A.z[X.e0[i >> 2] + (i & 3)] = zi;
+      return ri * zi;
+    });
+    ok = exchange<1, FUSE>(S, A, X.rows, ++epoch, tot);
+    if (threadIdx.x < 32) {
+      const double di = tot[0];
+      beta = di * rd;
+      d = di;
+      ++iter;
+      if (threadIdx.x == 0) {
+        int f = 0;
+        if (!(fabs(di) >= far) && sqrt(fabs(di)) < conv) f = 1;
+        else if (!isfinite(di)) f = 3;
+        else if (iter >= maxit) f = 2;
+        S.flag = f;
+        S.scal[0] = beta;
+        if (!ok) S.stop = ks->fault = 1;
+      }
+    }
+    COOP_SYNC();
+    if (S.flag) break;
+    const double be = S.scal[0];
+    double* to = FUSE ? po : A.p;
+    for (int i = threadIdx.x; i < X.rows; i += kCoopThreads) {
+      const double pi = X.q[i] + be * X.p[i];
+      X.p[i] = pi;
+      if ((i & 3) < (X.dw[i >> 2] & 7)) to[X.e0[i >> 2] + (i & 3)] = pi;
+    }
+    if (FUSE) {
+      __syncthreads();  // z in X.q is read: the product overwrites it
+      coop_spmv<L, true>(X, val, P.cols, pn, A.z, be);
+      to = pn;
+      pn = po;
+      po = to;
+    } else {
+      ok = exchange<0>(S, A, X.rows, ++epoch, tot);
+      if (threadIdx.x == 0 && !ok) S.stop = ks->fault = 1;
+      COOP_SYNC();
+      coop_spmv<L, false>(X, val, P.cols, A.p, nullptr, 0.0);
+    }
+    if (threadIdx.x < 32) rd = recip(d);
+  }
+  for (int i = threadIdx.x; i < X.rows; i += kCoopThreads)
+    if ((i & 3) < (X.dw[i >> 2] & 7)) A.x[X.e0[i >> 2] + (i & 3)] = X.x[i];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ks->d = d;
+    ks->pq = pq;
+    ks->alpha = alpha;
+    ks->beta = beta;
+    ks->iter = iter;
+    ks->conv_flag = S.flag;
+    ks->done = 1;
+  }
+}
+
+// rpsqmr: p = the direction q of the method, q = t = A q, d = d; k_sqmr_init's
+// start.  (r, M r) is summed with ||r||^2, so an iteration has PCG's exchanges.
+template <int L, bool FUSE>
+__global__ void __launch_bounds__(kCoopThreads, 1)
+    k_sqmr_coop(PanelView P, const double* __restrict__ val, CoopArgs A) {
+  extern __shared__ double coop_dyn[];
+  __shared__ CoopShared S;
+  const CoopLocal X = coop_setup<L>(P, A, true, coop_dyn);
+  KrylovScalars* ks = A.ks;
+  const double conv = ks->conv;
+  const int maxit = ks->maxit;
+  double rho = ks->d, tau = ks->normr, vj = ks->neta, nr = 0.0, sigma = 0.0, alpha = 0.0;
+  double rrho = 1.0 / rho, rtau = 1.0 / tau;
+  unsigned long long epoch = A.epoch;
+  int iter = 0;
+  double *pn = A.p, *po = A.p2;
+  // both values of the second exchange in slots apart from the one-value ones
+  CoopArgs A2 = A;
+  A2.slots = A.slots + 2 * (size_t)kReplicas * kCoopMaxCtas;
+  if (threadIdx.x == 0) S.stop = 0;
+  __syncthreads();
+  coop_spmv<L, false>(X, val, P.cols, A.p, nullptr, 0.0);
+  for (;;) {
+    __syncthreads();
+    coop_terms(S.part[0], X.rows, [&](int i) { return X.p[i] * X.q[i]; });
+    double tot1[1];
+    bool ok = exchange<1>(S, A, X.rows, ++epoch, tot1);
+    if (threadIdx.x < 32) {
+      sigma = tot1[0];
+      alpha = quotient(rho, sigma);
+      if (threadIdx.x == 0) {
+        S.scal[0] = alpha;
+        if (!ok) S.stop = ks->fault = 1;
+      }
+    }
+    COOP_SYNC();
+    const double al = S.scal[0];
+    if ((int)threadIdx.x < X.rows) {
+      double rr = 0.0, rt = 0.0;
+      for (int i = threadIdx.x; i < X.rows; i += kCoopThreads) {
+        const double ri = X.r[i] - al * X.q[i];
+        X.r[i] = ri;
+        const double ti = ri * X.m[i];
+        X.q[i] = ti;  // A q is done with: M r
+        if (FUSE && (i & 3) < (X.dw[i >> 2] & 7)) A.z[X.e0[i >> 2] + (i & 3)] = ti;
+        rr += ri * ri;
+        rt += ri * ti;
+      }
+      S.part[0][threadIdx.x] = rr;
+      S.part[1][threadIdx.x] = rt;
+    }
+    double tot[2];
+    ok = exchange<2, FUSE>(S, A2, X.rows, ++epoch, tot);
+    if (threadIdx.x < 32) {
+      nr = sqrt(tot[0]);
+      const double vn = nr * rtau;
+      const double cn2 = recip(1.0 + vn * vn);
+      tau = tau * vn * sqrt(cn2);
+      const double t1 = cn2 * vj * vj, t2 = cn2 * alpha, beta = tot[1] * rrho;
+      vj = vn;
+      ++iter;
+      if (threadIdx.x == 0) {
+        int f = 0;
+        if (sigma == 0.0 || !isfinite(alpha)) f = 3;
+        else if (nr < conv) f = 1;
+        else if (!isfinite(nr)) f = 3;
+        else if (iter >= maxit) f = 2;
+        else if (rho == 0.0) f = 3;
+        S.flag = f;
+        S.scal[1] = t1;
+        S.scal[2] = t2;
+        S.scal[3] = beta;
+        if (!ok) S.stop = ks->fault = 1;
+      }
+      rho = tot[1];
+    }
+    COOP_SYNC();
+    const double t1 = S.scal[1], t2 = S.scal[2], be = S.scal[3];
+    const bool go = S.flag == 0;
+    double* to = FUSE ? po : A.p;
+    for (int i = threadIdx.x; i < X.rows; i += kCoopThreads) {
+      const double qi = X.p[i], di = t1 * X.d[i] + t2 * qi;
+      X.d[i] = di;
+      X.x[i] = X.x[i] + di;
+      if (go) {
+        const double qn = X.q[i] + be * qi;
+        X.p[i] = qn;
+        if ((i & 3) < (X.dw[i >> 2] & 7)) to[X.e0[i >> 2] + (i & 3)] = qn;
+      }
+    }
+    if (!go) break;
+    if (FUSE) {
+      __syncthreads();
+      coop_spmv<L, true>(X, val, P.cols, pn, A.z, be);
+      to = pn;
+      pn = po;
+      po = to;
+    } else {
+      ok = exchange<0>(S, A, X.rows, ++epoch, tot1);
+      if (threadIdx.x == 0 && !ok) S.stop = ks->fault = 1;
+      COOP_SYNC();
+      coop_spmv<L, false>(X, val, P.cols, A.p, nullptr, 0.0);
+    }
+    if (threadIdx.x < 32) {
+      rrho = recip(rho);
+      rtau = recip(tau);
+    }
+  }
+  for (int i = threadIdx.x; i < X.rows; i += kCoopThreads)
+    if ((i & 3) < (X.dw[i >> 2] & 7)) A.x[X.e0[i >> 2] + (i & 3)] = X.x[i];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ks->d = rho;
+    ks->pq = sigma;
+    ks->normr = tau;
+    ks->neta = vj;
+    ks->ro1 = nr;
+    ks->iter = iter;
+    ks->conv_flag = S.flag;
+    ks->done = 1;
+  }
+}
+#undef COOP_SYNC
+
+template <bool SQMR, int L, bool FUSE>
+cudaError_t launch(const PanelView& P, const double* val, CoopArgs A, int grid, cudaStream_t s) {
+  constexpr int NPW = 32 / L;
+  const int groups = (P.nact + NPW - 1) / NPW;
+  A.nloc = NPW * ((groups + grid - 1) / grid);
+  const int smem = coop_local_bytes(SQMR, A.nloc);
+  const void* k = SQMR ? (const void*)k_sqmr_coop<L, FUSE> : (const void*)k_pcg_coop<L, FUSE>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  void* args[] = {(void*)&P, (void*)&val, (void*)&A};
+  return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kCoopThreads), args, smem, s);
+}
+
+// Two forms.  Up to 32 nodes per CTA: a warp per node and the exchange saved
+// by FUSE.  Above: two nodes per warp (fewer FP64 adds per node), where the
+// extra FP64 instruction per column costs more than the exchange.  Microseconds
+// per PCG iteration (fused warp per node / two nodes per warp / phase kernels):
+// column 2 x 2 x 40 10.0 / 14.3 / 25.7, cube 8^3 14.2 / 15.1 / 24.0, cube 12^3
+// 23.6 / 21.1 / 29.3, tetra 11^3 21.3 / 20.1 / 28.5.
+constexpr int kFuseNodes = 32;
+// Above this many panel values per CTA the FP64 pipe hides the phase kernels'
+// launches and feeds better from their many CTAs: cube 16^3 (70 k values per
+// CTA) 43.1 against 44.7 us, tetra 16^3 (61 k) 38.0 against 45.4, cube 20^3
+// (135 k) 83 against 68, tetra 20^3 (124 k) 81 against 79.
+constexpr int64_t kCoopValues = 80000;
+
+// at least a node per scheduler
+int coop_grid(const PanelView& P, int sms) {
+  return std::max(1, std::min({sms, kCoopMaxCtas, (P.nact + 3) / 4}));
+}
+
+}  // namespace
+
+size_t coop_scratch_bytes() {
+  return 6 * (size_t)kReplicas * kCoopMaxCtas * sizeof(Slot);
+}
+
+bool coop_fits(const PanelView& P, int64_t nnz, int sms) {
+  if (sms < 1 || P.nact < 1) return false;
+  const int grid = coop_grid(P, sms);
+  return nnz <= kCoopValues * grid &&
+         coop_local_bytes(true, 2 * (P.nact / (2 * grid) + 1)) <= kCoopMaxSmem;
+}
+
+cudaError_t krylov_coop(bool sqmr, const PanelView& P, const double* val, const double* m,
+                        KrylovVecs& V, KrylovScalars* ks, void* scratch,
+                        unsigned long long epoch, int sms, cudaStream_t s) {
+  const cudaError_t e = cudaMemsetAsync(&ks->fault, 0, sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  CoopArgs A{};
+  A.m = m;
+  A.x = V.x;
+  A.r = V.r;
+  A.p = V.p;
+  A.p2 = V.q;
+  A.z = V.z;
+  A.ks = ks;
+  A.slots = static_cast<Slot*>(scratch);
+  A.epoch = epoch;
+  const int grid = coop_grid(P, sms);
+  if (P.nact <= kFuseNodes * grid)
+    return sqmr ? launch<true, 32, true>(P, val, A, grid, s)
+                : launch<false, 32, true>(P, val, A, grid, s);
+  return sqmr ? launch<true, 16, false>(P, val, A, grid, s)
+              : launch<false, 16, false>(P, val, A, grid, s);
+}
+
+}  // namespace pm

@@ -156,6 +156,7 @@ struct Dev {
   unsigned* counter = nullptr;
   double* norms = nullptr;
   int* err = nullptr;
+  void* coop = nullptr;  // exchange slots of the cooperative solve
   int* trips = nullptr;  // trips of the device-side solve loop (pcg_loop)
 };
 
@@ -222,6 +223,9 @@ struct Handle {
   // driver cannot build it)
   cudaGraphExec_t pcg_loop = nullptr;
   bool pcg_loop_failed = false;
+  int sms = 0;                 // SMs of the handle's device
+  unsigned long long coop_epoch = 0;  // the slots' last epoch
+  bool coop_failed = false;    // the cooperative solve was refused or gave up once
   // a batch time step as one graph (step_batch_graph): control state and
   // per-instance arrays on the device, the executable graph of the last step
   pm::BatchCtl* d_bctl = nullptr;

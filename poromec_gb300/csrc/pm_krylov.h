@@ -112,6 +112,7 @@ struct KrylovScalars {
   int iter;       // iterations completed (all restarts)
   int jcycle;     // iterations of the current MINRES cycle
   int maxit;
+  int fault;      // a wait of the cooperative solve gave up: its result is void
 };
 
 struct KrylovVecs {
@@ -150,6 +151,19 @@ cudaError_t sqmr_init(int n, const double* b, const double* m, KrylovVecs& V, fl
 cudaError_t sqmr_iteration(const PanelView& P, const double* val64, int n, const double* m,
                            KrylovVecs& V, KrylovScalars* ks, double* partial,
                            unsigned* counter, cudaStream_t s);
+// A whole FP64 PCG (rpsqmr) solve after pcg_init (sqmr_init) as one cooperative
+// kernel (pm_coop.cu) on at most sms CTAs.  scratch holds coop_scratch_bytes(),
+// zero before its first use; epoch is larger than any the earlier solves on it
+// reached (kCoopEpochs per iteration).
+// The flags are in *ks; ks->fault set or conv_flag 0: not solved.
+// coop_fits: whether this form is the faster one for a mesh of nnz panel values.
+constexpr int kCoopMaxSmem = 200 * 1024;
+constexpr int kCoopEpochs = 3;
+size_t coop_scratch_bytes();
+bool coop_fits(const PanelView& P, int64_t nnz, int sms);
+cudaError_t krylov_coop(bool sqmr, const PanelView& P, const double* val, const double* m,
+                        KrylovVecs& V, KrylovScalars* ks, void* scratch,
+                        unsigned long long epoch, int sms, cudaStream_t s);
 // GMRES(l) vector kernels (pm_gmres.cu)
 cudaError_t gm_resid(int n, const double* b, const double* ax, const double* m, double* g1,
                      double* out, double* partial, unsigned* counter, cudaStream_t s);
