@@ -1,6 +1,7 @@
 // pm_elements.cu -- element kernels of the Biot hot path on sm_103a.
 //
-// One CTA per element (64 threads for hexa20, 32 for tetra10).  Phase 1 maps
+// One CTA per element (64 threads for hexa20, 32 for tetra10; the hexa20
+// matrix, in pm_hexa_mma.h, 256).  Phase 1 maps
 // the integration points to threads: each thread builds the subparametric
 // geometry of its point (vertex Jacobian, determinant, inverse; the
 // quadratic derivatives mapped with that same inverse, as jacob3d_m does in
@@ -18,13 +19,12 @@
 // products, summed in a different order).  The blocks are added straight
 // into the node panels; elements of one colour share no node, so the adds
 // need no atomics.  The hexa's shape functions at its 64 points come from a
-// table filled once per device (ensure_shape_tables); each point's values
-// are scaled by sqrt(w_g) before the pair loops, so these need no w_g.
+// table filled once per device (ensure_shape_tables).
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <mutex>
-#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -385,36 +385,27 @@ __device__ __forceinline__ int eq_of(const ElemLaunch& L, int n, int k) {
   return L.eq[(size_t)kNdf * (n - 1) + k];
 }
 
-template <typename T>
-__device__ __forceinline__ void add_val(double* v64, float* v32, int64_t a, T v) {
-  if (v64) v64[a] += double(v);
-  else v32[a] += float(v);
+// (the entry is rounded before the add: the same panels with and without RHS)
+__device__ __forceinline__ void add_val(double* val, int64_t a, double v) {
+  val[a] = __dadd_rn(val[a], v);
 }
 
-// ---------------------------------------------------------------------------
-// isw = 2, lhs: element matrix into the panels.
-// ---------------------------------------------------------------------------
-// The weight a pair loop still applies at point gq: none for the hexa, whose
-// point values k_assemble_K scales by sqrt(w); w for the tetra.
-template <bool HEXA, typename T>
-__device__ __forceinline__ T pair_weight(const Geo<HEXA, T>& G, int gq) {
-  if constexpr (HEXA) return T(1);
-  else return G.w[gq];
-}
+#include "pm_hexa_mma.h"
 
-template <bool HEXA, typename T>
+// ---------------------------------------------------------------------------
+// isw = 2, lhs: element matrix into the panels (tetra10).
+// ---------------------------------------------------------------------------
 struct SmK {
-  static constexpr int NEN = ET<HEXA>::NEN, NV = ET<HEXA>::NV, NST = 3 * NEN + NV,
+  static constexpr int NEN = ET<false>::NEN, NV = ET<false>::NV, NST = 3 * NEN + NV,
                        NSLOT = NEN + NV;
-  Geo<HEXA, T> G;
+  Geo<false, double> G;
   ElemCtx E;
   int sEq[NEN][kNdf];  // equation numbers of the local dofs
   int sE0[NEN];        // first equation of each node
   int sFail;
-  // with RHS: the element's dof values, and (tetra) the contribution slots;
-  // the hexa's slots reuse G.g once the pair loops have read it
+  // with RHS: the element's dof values and the contribution slots
   double ul[NST];
-  double Cx[HEXA ? 1 : NST * NSLOT];
+  double Cx[NST * NSLOT];
 };
 
 // Element matrix into the panels; with RHS also b -= K_e u_e from the same
@@ -423,18 +414,16 @@ struct SmK {
 // is deterministic: every block writes its share of a row into a slot of its
 // own (row r of the element vector: slot j for node j's u columns, slot
 // NEN + l for vertex l's p column) and each row sums its slots in order.
-template <bool HEXA, typename T, bool RHS>
-__global__ void __launch_bounds__(ET<HEXA>::NT)
-    k_assemble_K(ElemLaunch L, double* val64, float* val32, const double* __restrict__ u,
-                 double* __restrict__ bvec) {
-  constexpr int NEN = ET<HEXA>::NEN, NV = ET<HEXA>::NV, NGP = ET<HEXA>::NGP,
-                NT = ET<HEXA>::NT;
-  constexpr int NST = SmK<HEXA, T>::NST, NSLOT = SmK<HEXA, T>::NSLOT;
-  static_assert(!RHS || std::is_same<T, double>::value, "the fused product is FP64");
-  static_assert(!HEXA || NST * NSLOT <= NGP * NEN * 3, "hexa slots fit in G.g");
+template <bool RHS>
+__global__ void __launch_bounds__(ET<false>::NT)
+    k_assemble_tetra(ElemLaunch L, double* val, const double* __restrict__ u,
+                     double* __restrict__ bvec) {
+  constexpr int NEN = ET<false>::NEN, NV = ET<false>::NV, NGP = ET<false>::NGP,
+                NT = ET<false>::NT;
+  constexpr int NST = SmK::NST, NSLOT = SmK::NSLOT;
   extern __shared__ __align__(16) unsigned char smem[];
-  SmK<HEXA, T>& S = *reinterpret_cast<SmK<HEXA, T>*>(smem);
-  Geo<HEXA, T>& G = S.G;
+  SmK& S = *reinterpret_cast<SmK*>(smem);
+  Geo<false, double>& G = S.G;
   ElemCtx& E = S.E;
   auto& sEq = S.sEq;
   auto& sE0 = S.sE0;
@@ -442,7 +431,7 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
   const double* ul = S.ul;
   const int el = L.elems[blockIdx.x];
   if (threadIdx.x == 0) sFail = 0;
-  load_element<HEXA, T>(L, el, E, G);
+  load_element<false, double>(L, el, E, G);
   for (int k = threadIdx.x; k < NEN; k += NT) {
     const int n = E.nodes[k];
     int e0 = 0x7fffffff;
@@ -460,40 +449,20 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
       S.ul[k] = u[(size_t)kNdf * (n - 1) + q];
     }
   }
-  for (int gq = threadIdx.x; gq < NGP; gq += NT) {
-    if (!point_geometry<HEXA, T>(G, gq, nullptr)) {
-      sFail = 1;
-      continue;
-    }
-    // every entry below is a sum over points of w times a product of two
-    // point values: for the hexa's 64 points, scale the point's values by
-    // sqrt(w) (w > 0 here) and the pair loops need no multiply by w; the
-    // tetra's 4-point loops keep the per-pair weight
-    if constexpr (HEXA) {
-      const T sw = sqrt(G.w[gq]);
-#pragma unroll
-      for (int k = 0; k < NEN; ++k) {
-        G.g[gq][k][0] *= sw; G.g[gq][k][1] *= sw; G.g[gq][k][2] *= sw;
-      }
-#pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        G.hp[gq][k] *= sw;
-        G.gp[gq][k][0] *= sw; G.gp[gq][k][1] *= sw; G.gp[gq][k][2] *= sw;
-      }
-    }
-  }
+  for (int gq = threadIdx.x; gq < NGP; gq += NT)
+    if (!point_geometry<false, double>(G, gq, nullptr)) sFail = 1;
   __syncthreads();
   if (sFail) {
     if (threadIdx.x == 0) atomicOr(L.err, 1);
     return;
   }
   const MatConst mc = L.mat[E.mat - 1];
-  const T a = T(mc.a), b = T(mc.b), c = T(mc.c);
+  const double a = mc.a, b = mc.b, c = mc.c;
   const int32_t* slot = L.slot + (size_t)NEN * NEN * blockIdx.x;
   // ---- Kuu: node pairs (i >= j) -------------------------------------------
   constexpr int NPAIR = NEN * (NEN + 1) / 2, QUU = (NPAIR + NT - 1) / NT;
   // RHS: per pair, row (i, k) gets K_ij u_j (slot j) and, for i != j, row
-  // (j, l) gets K_ij^T u_i (slot i); held here until G.g is free
+  // (j, l) gets K_ij^T u_i (slot i)
   double ru[RHS ? QUU : 1][6];
 #pragma unroll
   for (int q = 0; q < QUU; ++q) {
@@ -504,18 +473,18 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
     while ((i + 1) * (i + 2) / 2 <= pr) ++i;
     while (i * (i + 1) / 2 > pr) --i;
     const int j = pr - i * (i + 1) / 2;
-    T P[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    double P[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
 #pragma unroll 4
     for (int gq = 0; gq < NGP; ++gq) {
-      const T w = pair_weight(G, gq);
-      const T gi0 = w * G.g[gq][i][0], gi1 = w * G.g[gq][i][1], gi2 = w * G.g[gq][i][2];
-      const T gj0 = G.g[gq][j][0], gj1 = G.g[gq][j][1], gj2 = G.g[gq][j][2];
+      const double w = G.w[gq];
+      const double gi0 = w * G.g[gq][i][0], gi1 = w * G.g[gq][i][1], gi2 = w * G.g[gq][i][2];
+      const double gj0 = G.g[gq][j][0], gj1 = G.g[gq][j][1], gj2 = G.g[gq][j][2];
       P[0][0] += gi0 * gj0; P[0][1] += gi0 * gj1; P[0][2] += gi0 * gj2;
       P[1][0] += gi1 * gj0; P[1][1] += gi1 * gj1; P[1][2] += gi1 * gj2;
       P[2][0] += gi2 * gj0; P[2][1] += gi2 * gj1; P[2][2] += gi2 * gj2;
     }
-    const T tr = P[0][0] + P[1][1] + P[2][2];
-    T K[3][3];
+    const double tr = P[0][0] + P[1][1] + P[2][2];
+    double K[3][3];
 #pragma unroll
     for (int k = 0; k < 3; ++k)
 #pragma unroll
@@ -542,17 +511,16 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
       for (int l = 0; l < 3; ++l) {
         const int ec = sEq[j][l];
         if (ec == 0) continue;
-        add_val<T>(val64, val32, rowi + ec, K[k][l]);
+        add_val(val, rowi + ec, K[k][l]);
         if (i != j) {
           // transposed entry in node j's panel: row ec, column er
-          add_val<T>(val64, val32,
-                     offj + (int64_t)(ec - sE0[j]) * Wj + sji - sE0[i] + er, K[k][l]);
+          add_val(val, offj + (int64_t)(ec - sE0[j]) * Wj + sji - sE0[i] + er, K[k][l]);
         }
       }
     }
   }
   // ---- Kpu / Kup: (vertex l, node j) ---------------------------------------
-  const T alpha = T(mc.coef_biot);
+  const double alpha = mc.coef_biot;
   constexpr int NPU = NV * NEN, QPU = (NPU + NT - 1) / NT;
   // RHS: p row l gets Kpu_lj . u_j (slot j), rows (j, k) get Kup_jl p_l
   // (slot NEN + l)
@@ -562,13 +530,13 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
     const int pr = threadIdx.x + q * NT;
     if (pr >= NPU) break;
     const int l = pr / NEN, j = pr % NEN;
-    T A0 = 0, A1 = 0, A2 = 0;
+    double A0 = 0, A1 = 0, A2 = 0;
 #pragma unroll 4
     for (int gq = 0; gq < NGP; ++gq) {
-      const T wh = pair_weight(G, gq) * G.hp[gq][l];
+      const double wh = G.w[gq] * G.hp[gq][l];
       A0 += wh * G.g[gq][j][0]; A1 += wh * G.g[gq][j][1]; A2 += wh * G.g[gq][j][2];
     }
-    const T Kv[3] = {-alpha * A0, -alpha * A1, -alpha * A2};
+    const double Kv[3] = {-alpha * A0, -alpha * A1, -alpha * A2};
     if constexpr (RHS) {
       const double pl = ul[3 * NEN + l];
       rk[q][0] = Kv[0] * ul[3 * j] + Kv[1] * ul[3 * j + 1] + Kv[2] * ul[3 * j + 2];
@@ -584,16 +552,13 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
     for (int k = 0; k < 3; ++k) {
       const int ec = sEq[j][k];
       if (ec == 0) continue;
-      add_val<T>(val64, val32, offl + (int64_t)(er - sE0[l]) * Wl + slj - sE0[j] + ec, Kv[k]);
-      add_val<T>(val64, val32, offj + (int64_t)(ec - sE0[j]) * Wj + sjl - sE0[l] + er, Kv[k]);
+      add_val(val, offl + (int64_t)(er - sE0[l]) * Wl + slj - sE0[j] + ec, Kv[k]);
+      add_val(val, offj + (int64_t)(ec - sE0[j]) * Wj + sjl - sE0[l] + er, Kv[k]);
     }
   }
   double* C = nullptr;
   if constexpr (RHS) {
-    // every read of G.g is done: the hexa's slots may overwrite it
-    __syncthreads();
-    if constexpr (HEXA) C = reinterpret_cast<double*>(&G.g[0][0][0]);
-    else C = S.Cx;
+    C = S.Cx;
 #pragma unroll
     for (int q = 0; q < QUU; ++q) {
       const int pr = threadIdx.x + q * NT;
@@ -619,27 +584,20 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
     }
   }
   // ---- Kpp: vertex pairs (l >= m) ------------------------------------------
-  const T imod = T(mc.imod_biot), dtp = T(mc.perm * L.dt);
+  const double imod = mc.imod_biot, dtp = mc.perm * L.dt;
   constexpr int NPP = NV * (NV + 1) / 2;
   for (int pr = threadIdx.x; pr < NPP; pr += NT) {
     int l = 0;
     while ((l + 1) * (l + 2) / 2 <= pr) ++l;
     const int m = pr - l * (l + 1) / 2;
-    T acc = 0, am = 0, ak = 0;
+    double acc = 0;
 #pragma unroll 4
     for (int gq = 0; gq < NGP; ++gq) {
-      if constexpr (HEXA) {  // values carry sqrt(w)
-        am += G.hp[gq][l] * G.hp[gq][m];
-        ak += G.gp[gq][l][0] * G.gp[gq][m][0] + G.gp[gq][l][1] * G.gp[gq][m][1] +
-              G.gp[gq][l][2] * G.gp[gq][m][2];
-      } else {
-        const T w = G.w[gq];
-        acc += w * imod * G.hp[gq][l] * G.hp[gq][m] +
-               w * dtp * (G.gp[gq][l][0] * G.gp[gq][m][0] + G.gp[gq][l][1] * G.gp[gq][m][1] +
-                          G.gp[gq][l][2] * G.gp[gq][m][2]);
-      }
+      const double w = G.w[gq];
+      acc += w * imod * G.hp[gq][l] * G.hp[gq][m] +
+             w * dtp * (G.gp[gq][l][0] * G.gp[gq][m][0] + G.gp[gq][l][1] * G.gp[gq][m][1] +
+                        G.gp[gq][l][2] * G.gp[gq][m][2]);
     }
-    if constexpr (HEXA) acc = imod * am + dtp * ak;
     if constexpr (RHS) {
       C[(3 * NEN + l) * NSLOT + NEN + m] = -acc * ul[3 * NEN + m];
       if (l != m) C[(3 * NEN + m) * NSLOT + NEN + l] = -acc * ul[3 * NEN + l];
@@ -647,12 +605,10 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
     const int er = sEq[l][3], ec = sEq[m][3];
     if (er == 0 || ec == 0) continue;
     const int nl = E.nodes[l], nm = E.nodes[m];
-    add_val<T>(val64, val32,
-               L.node_val_off[nl - 1] + (int64_t)(er - sE0[l]) * L.node_W[nl - 1] +
+    add_val(val, L.node_val_off[nl - 1] + (int64_t)(er - sE0[l]) * L.node_W[nl - 1] +
                    slot[l * NEN + m] - sE0[m] + ec, -acc);
     if (l != m)
-      add_val<T>(val64, val32,
-                 L.node_val_off[nm - 1] + (int64_t)(ec - sE0[m]) * L.node_W[nm - 1] +
+      add_val(val, L.node_val_off[nm - 1] + (int64_t)(ec - sE0[m]) * L.node_W[nm - 1] +
                      slot[m * NEN + l] - sE0[l] + er, -acc);
   }
   if constexpr (RHS) {
@@ -1424,7 +1380,7 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
 // opt-in above 48 KB set once per kernel.
 template <typename Sm, typename Kern, typename... Args>
 cudaError_t launch_elem(Kern k, int n, int nt, cudaStream_t s, Args... args) {
-  // kernels of one signature and shared-memory struct (k_assemble_K with and
+  // kernels of one signature and shared-memory struct (an assembly with and
   // without the fused product) share this instantiation: key on the kernel
   static std::mutex mu;
   static std::vector<std::pair<const void*, int>> opted;
@@ -1469,21 +1425,16 @@ cudaError_t ensure_shape_tables() {
 cudaError_t launch_assemble_K(const ElemLaunch& L, bool hexa, double* val, cudaStream_t s,
                               const double* u, double* b) {
   if (L.nelem <= 0) return cudaSuccess;
-  float* no32 = nullptr;
   if (b) {
     if (hexa)
-      return launch_elem<SmK<true, double>>(k_assemble_K<true, double, true>, L.nelem, 64, s,
-                                            L, val, no32, u, b);
-    return launch_elem<SmK<false, double>>(k_assemble_K<false, double, true>, L.nelem, 32, s,
-                                           L, val, no32, u, b);
+      return launch_elem<SmHx>(k_assemble_hexa<true>, L.nelem, kHxThreads, s, L, val, u, b);
+    return launch_elem<SmK>(k_assemble_tetra<true>, L.nelem, 32, s, L, val, u, b);
   }
   const double* nu = nullptr;
   double* nb = nullptr;
   if (hexa)
-    return launch_elem<SmK<true, double>>(k_assemble_K<true, double, false>, L.nelem, 64, s, L,
-                                          val, no32, nu, nb);
-  return launch_elem<SmK<false, double>>(k_assemble_K<false, double, false>, L.nelem, 32, s, L,
-                                         val, no32, nu, nb);
+    return launch_elem<SmHx>(k_assemble_hexa<false>, L.nelem, kHxThreads, s, L, val, nu, nb);
+  return launch_elem<SmK>(k_assemble_tetra<false>, L.nelem, 32, s, L, val, nu, nb);
 }
 
 cudaError_t launch_residual(const ElemLaunch& L, bool hexa, const double* u,
