@@ -1,9 +1,9 @@
 // pm_elements.cu -- element kernels of the Biot hot path on sm_103a.
 //
-// One CTA per element (64 threads for hexa20, 32 for tetra10; the hexa20
-// matrix, in pm_hexa_mma.h, 256).  Phase 1 maps
-// the integration points to threads: each thread builds the subparametric
-// geometry of its point (vertex Jacobian, determinant, inverse; the
+// One CTA per element (32 threads for tetra10, 64 for hexa20; the hexa20 matrix,
+// in pm_hexa_mma.h, 256, and its matrix-free passes, in pm_hexa_sum.h, 192).
+// Phase 1 maps the integration points to threads: each thread builds the
+// subparametric geometry of its point (vertex Jacobian, determinant, inverse; the
 // quadratic derivatives mapped with that same inverse, as jacob3d_m does in
 // Elmlib.f:2301-2396) into shared memory.  Phase 2 maps the element matrix
 // (or vector) entries to threads and reduces over the points.
@@ -133,25 +133,6 @@ __device__ __forceinline__ void sf_hexa20_d(T r, T s, T t, T* hr, T* hs, T* ht) 
 }
 
 template <typename T>
-__device__ __forceinline__ void sf_hexa20_v(T r, T s, T t, T* h) {
-  const T pR = 1 + r, pS = 1 + s, pT = 1 + t, mR = 1 - r, mS = 1 - s, mT = 1 - t;
-  const T mRr = 1 - r * r, mSs = 1 - s * s, mTt = 1 - t * t;
-  const T e = T(0.125), q = T(0.25);
-  h[0] = pR * pS * pT * (r + s + t - 2) * e;
-  h[1] = mR * pS * pT * (-r + s + t - 2) * e;
-  h[2] = mR * mS * pT * (-r - s + t - 2) * e;
-  h[3] = pR * mS * pT * (r - s + t - 2) * e;
-  h[4] = pR * pS * mT * (r + s - t - 2) * e;
-  h[5] = mR * pS * mT * (-r + s - t - 2) * e;
-  h[6] = mR * mS * mT * (-r - s - t - 2) * e;
-  h[7] = pR * mS * mT * (r - s - t - 2) * e;
-  h[8] = mRr * pS * pT * q; h[9] = mR * mSs * pT * q; h[10] = mRr * mS * pT * q;
-  h[11] = pR * mSs * pT * q; h[12] = mRr * pS * mT * q; h[13] = mR * mSs * mT * q;
-  h[14] = mRr * mS * mT * q; h[15] = pR * mSs * mT * q; h[16] = pR * pS * mTt * q;
-  h[17] = mR * pS * mTt * q; h[18] = mR * mS * mTt * q; h[19] = pR * mS * mTt * q;
-}
-
-template <typename T>
 __device__ __forceinline__ void sf_tetra4(T r, T s, T t, T* h, T* hr, T* hs, T* ht) {
   h[0] = r; h[1] = s; h[2] = t; h[3] = 1 - r - s - t;
   hr[0] = 1; hr[1] = 0; hr[2] = 0; hr[3] = -1;
@@ -197,8 +178,7 @@ struct Geo {
 // holds one function at the 64 points, so a warp's loads are coalesced.
 constexpr int kTabH8 = 0;     // rows 0..31: h, hr, hs, ht of sfhexa8 (8 each)
 constexpr int kTabH20D = 32;  // rows 32..91: hr, hs, ht of sfhexa20 (20 each)
-constexpr int kTabH20V = 92;  // rows 92..111: h of sfhexa20
-constexpr int kTabRows = 112;
+constexpr int kTabRows = 92;
 constexpr int kHexaGp = 64;
 __device__ double gShapeHexa[kTabRows * kHexaGp];
 
@@ -207,10 +187,9 @@ __global__ void k_fill_shape_tables() {
   if (gq >= kHexaGp) return;
   const int lz = gq >> 4, ly = (gq >> 2) & 3, lx = gq & 3;
   const double r = cPG4[lx], s = cPG4[ly], t = cPG4[lz];
-  double h[8], hr[8], hs[8], ht[8], ur[20], us[20], ut[20], hv[20];
+  double h[8], hr[8], hs[8], ht[8], ur[20], us[20], ut[20];
   sf_hexa8<double>(r, s, t, h, hr, hs, ht);
   sf_hexa20_d<double>(r, s, t, ur, us, ut);
-  sf_hexa20_v<double>(r, s, t, hv);
   double* tb = gShapeHexa + gq;
   for (int k = 0; k < 8; ++k) {
     tb[(kTabH8 + k) * kHexaGp] = h[k];
@@ -222,7 +201,6 @@ __global__ void k_fill_shape_tables() {
     tb[(kTabH20D + k) * kHexaGp] = ur[k];
     tb[(kTabH20D + 20 + k) * kHexaGp] = us[k];
     tb[(kTabH20D + 40 + k) * kHexaGp] = ut[k];
-    tb[(kTabH20V + k) * kHexaGp] = hv[k];
   }
 }
 
@@ -235,7 +213,7 @@ __device__ bool point_geometry_rst(Geo<HEXA, T>& G, int gq, T r, T s, T t, T wq,
 // vertices, its inverse by one reciprocal of the determinant, and the
 // physical derivatives, with the table rows streamed from L1.
 template <typename T>
-__device__ bool point_geometry_hexa_tab(Geo<true, T>& G, int gq, T* huv) {
+__device__ bool point_geometry_hexa_tab(Geo<true, T>& G, int gq) {
   constexpr int NEN = 20, NV = 8;
   const double* tb = gShapeHexa + gq;
   auto tab = [tb](int row) { return T(__ldg(tb + row * kHexaGp)); };
@@ -284,15 +262,13 @@ __device__ bool point_geometry_hexa_tab(Geo<true, T>& G, int gq, T* huv) {
     G.g[gq][k][1] = Ji[1][0] * ur + Ji[1][1] * us + Ji[1][2] * ut;
     G.g[gq][k][2] = Ji[2][0] * ur + Ji[2][1] * us + Ji[2][2] * ut;
   }
-  if (huv)
-    for (int k = 0; k < NEN; ++k) huv[k] = tab(kTabH20V + k);
   return true;
 }
 
 template <bool HEXA, typename T>
 __device__ bool point_geometry(Geo<HEXA, T>& G, int gq, T* huv) {
   if constexpr (HEXA) {
-    return point_geometry_hexa_tab<T>(G, gq, huv);
+    return point_geometry_hexa_tab<T>(G, gq);
   } else {
     return point_geometry_rst<HEXA, T>(G, gq, T(cPRI4[gq]), T(cPSI4[gq]), T(cPTI4[gq]),
                                        T(0.25), huv);
@@ -351,10 +327,8 @@ __device__ bool point_geometry_rst(Geo<HEXA, T>& G, int gq, T r, T s, T t, T wq,
     G.g[gq][k][1] = Ji[1][0] * ur[k] + Ji[1][1] * us[k] + Ji[1][2] * ut[k];
     G.g[gq][k][2] = Ji[2][0] * ur[k] + Ji[2][1] * us[k] + Ji[2][2] * ut[k];
   }
-  if (huv) {
-    if (HEXA) sf_hexa20_v<T>(r, s, t, huv);
-    else sf_tetra10_v<T>(r, s, t, huv);
-  }
+  if constexpr (!HEXA)
+    if (huv) sf_tetra10_v<T>(r, s, t, huv);
   return true;
 }
 
@@ -629,24 +603,22 @@ __global__ void __launch_bounds__(ET<false>::NT)
 //   p rows: -w [ alpha Np_l div u + Np_l (Np . u_p)/M + dt perm grad Np_l . grad p ]
 // with sigma = stress3d(deform3d(u)) -- the rows of s.u in lku_m.
 // ---------------------------------------------------------------------------
-template <bool HEXA>
 struct SmR {
-  Geo<HEXA, double> G;
-  double ul[3 * ET<HEXA>::NEN + ET<HEXA>::NV];
-  double S6[ET<HEXA>::NGP][6];  // w (sigma - alpha p I)
-  double Q4[ET<HEXA>::NGP][4];  // w (alpha div + p/M), w dt perm grad p
+  Geo<false, double> G;
+  double ul[3 * ET<false>::NEN + ET<false>::NV];
+  double S6[ET<false>::NGP][6];  // w (sigma - alpha p I)
+  double Q4[ET<false>::NGP][4];  // w (alpha div + p/M), w dt perm grad p
   ElemCtx E;
   int sFail;
 };
 
-template <bool HEXA>
-__global__ void __launch_bounds__(ET<HEXA>::NT)
-    k_residual(ElemLaunch L, const double* __restrict__ u, double* __restrict__ bvec) {
-  constexpr int NEN = ET<HEXA>::NEN, NV = ET<HEXA>::NV, NGP = ET<HEXA>::NGP,
-                NT = ET<HEXA>::NT, NST = 3 * NEN + NV;
+__global__ void __launch_bounds__(ET<false>::NT)
+    k_residual_tetra(ElemLaunch L, const double* __restrict__ u, double* __restrict__ bvec) {
+  constexpr int NEN = ET<false>::NEN, NV = ET<false>::NV, NGP = ET<false>::NGP,
+                NT = ET<false>::NT, NST = 3 * NEN + NV;
   extern __shared__ __align__(16) unsigned char smem[];
-  SmR<HEXA>& S = *reinterpret_cast<SmR<HEXA>*>(smem);
-  Geo<HEXA, double>& G = S.G;
+  SmR& S = *reinterpret_cast<SmR*>(smem);
+  Geo<false, double>& G = S.G;
   ElemCtx& E = S.E;
   auto& ul = S.ul;
   auto& S6 = S.S6;
@@ -654,7 +626,7 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
   int& sFail = S.sFail;
   const int el = L.elems[blockIdx.x];
   if (threadIdx.x == 0) sFail = 0;
-  load_element<HEXA, double>(L, el, E, G);
+  load_element<false, double>(L, el, E, G);
   for (int k = threadIdx.x; k < NST; k += NT) {
     const int n = k < 3 * NEN ? E.nodes[k / 3] : E.nodes[k - 3 * NEN];
     const int q = k < 3 * NEN ? k % 3 : 3;
@@ -663,7 +635,7 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
   __syncthreads();
   const MatConst mc = L.mat[E.mat - 1];
   for (int gq = threadIdx.x; gq < NGP; gq += NT) {
-    if (!point_geometry<HEXA, double>(G, gq, nullptr)) {
+    if (!point_geometry<false, double>(G, gq, nullptr)) {
       sFail = 1;
       continue;
     }
@@ -911,31 +883,29 @@ __device__ void face_loads(const ElemLaunch& L, const int* iqm, const int* iqh,
   }
 }
 
-template <bool HEXA>
 struct SmF {
-  Geo<HEXA, double> G;
-  double ul[3 * ET<HEXA>::NEN + ET<HEXA>::NV];
-  double dpl[ET<HEXA>::NV];
-  double S6[ET<HEXA>::NGP][6];
-  double Q4[ET<HEXA>::NGP][4];
-  double HU[ET<HEXA>::NGP][ET<HEXA>::NEN];  // w pm_d N_i
-  double pf[3 * ET<HEXA>::NEN + ET<HEXA>::NV];  // face-load contributions
+  Geo<false, double> G;
+  double ul[3 * ET<false>::NEN + ET<false>::NV];
+  double dpl[ET<false>::NV];
+  double S6[ET<false>::NGP][6];
+  double Q4[ET<false>::NGP][4];
+  double HU[ET<false>::NGP][ET<false>::NEN];  // w pm_d N_i
+  double pf[3 * ET<false>::NEN + ET<false>::NV];  // face-load contributions
   ElemCtx E;
   int iqm[7], iqh[7];
   int sFail, sAny;
 };
 
-template <bool HEXA>
-__global__ void __launch_bounds__(ET<HEXA>::NT)
-    k_rhs4(ElemLaunch L, const double* __restrict__ u, const double* __restrict__ dp,
+__global__ void __launch_bounds__(ET<false>::NT)
+    k_rhs4_tetra(ElemLaunch L, const double* __restrict__ u, const double* __restrict__ dp,
            const int32_t* __restrict__ eload, const int32_t* __restrict__ eloadp,
            const int32_t* __restrict__ load, const double* __restrict__ fload, int maxt,
            double* __restrict__ bvec) {
-  constexpr int NEN = ET<HEXA>::NEN, NV = ET<HEXA>::NV, NGP = ET<HEXA>::NGP,
-                NT = ET<HEXA>::NT, NST = 3 * NEN + NV;
+  constexpr int NEN = ET<false>::NEN, NV = ET<false>::NV, NGP = ET<false>::NGP,
+                NT = ET<false>::NT, NST = 3 * NEN + NV;
   extern __shared__ __align__(16) unsigned char smem[];
-  SmF<HEXA>& S = *reinterpret_cast<SmF<HEXA>*>(smem);
-  Geo<HEXA, double>& G = S.G;
+  SmF& S = *reinterpret_cast<SmF*>(smem);
+  Geo<false, double>& G = S.G;
   ElemCtx& E = S.E;
   auto& ul = S.ul;
   auto& dpl = S.dpl;
@@ -949,7 +919,7 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
   int& sAny = S.sAny;
   const int el = L.elems[blockIdx.x];
   if (threadIdx.x == 0) { sFail = 0; sAny = 0; }
-  load_element<HEXA, double>(L, el, E, G);
+  load_element<false, double>(L, el, E, G);
   for (int k = threadIdx.x; k < NST; k += NT) {
     const int n = k < 3 * NEN ? E.nodes[k / 3] : E.nodes[k - 3 * NEN];
     const int q = k < 3 * NEN ? k % 3 : 3;
@@ -966,7 +936,7 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
   const MatConst mc = L.mat[E.mat - 1];
   for (int gq = threadIdx.x; gq < NGP; gq += NT) {
     double huv[NEN];
-    if (!point_geometry<HEXA, double>(G, gq, huv)) {
+    if (!point_geometry<false, double>(G, gq, huv)) {
       sFail = 1;
       continue;
     }
@@ -1008,7 +978,7 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
   __syncthreads();
   if (sAny && threadIdx.x == 0) {
     int f = 0;
-    face_loads<HEXA>(L, iqm, iqh, G.xv, load, fload, maxt, pf, &f);
+    face_loads<false>(L, iqm, iqh, G.xv, load, fload, maxt, pf, &f);
     if (f) sFail = 1;
   }
   __syncthreads();
@@ -1064,33 +1034,32 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
 //   d/dlog M:   lam_p^T Kstor du_p,  Kstor = -(1/M) int(N N)
 //   accumulated into grad[3 (el - 1) + {0, 1, 2}].
 // ---------------------------------------------------------------------------
-template <bool HEXA>
 struct SmA {
-  Geo<HEXA, double> G;
-  double ll[3 * ET<HEXA>::NEN + ET<HEXA>::NV];  // lam on the element dofs
-  double ul[3 * ET<HEXA>::NEN + ET<HEXA>::NV];  // u_n (MODE 1)
-  double dl[ET<HEXA>::NV];                      // du_p (MODE 1)
-  double S6[ET<HEXA>::NGP][6];
-  double Q4[ET<HEXA>::NGP][4];
-  double gsum[3][ET<HEXA>::NT / 32];
+  Geo<false, double> G;
+  double ll[3 * ET<false>::NEN + ET<false>::NV];  // lam on the element dofs
+  double ul[3 * ET<false>::NEN + ET<false>::NV];  // u_n (MODE 1)
+  double dl[ET<false>::NV];                      // du_p (MODE 1)
+  double S6[ET<false>::NGP][6];
+  double Q4[ET<false>::NGP][4];
+  double gsum[3][ET<false>::NT / 32];
   ElemCtx E;
   int sFail;
 };
 
-template <bool HEXA, int MODE>
-__global__ void __launch_bounds__(ET<HEXA>::NT)
-    k_adjoint(ElemLaunch L, const double* __restrict__ lam, const double* __restrict__ un,
+template <int MODE>
+__global__ void __launch_bounds__(ET<false>::NT)
+    k_adjoint_tetra(ElemLaunch L, const double* __restrict__ lam, const double* __restrict__ un,
               const double* __restrict__ dun, double* __restrict__ mu, double* __restrict__ nu,
               double* __restrict__ grad) {
-  constexpr int NEN = ET<HEXA>::NEN, NV = ET<HEXA>::NV, NGP = ET<HEXA>::NGP,
-                NT = ET<HEXA>::NT, NST = 3 * NEN + NV;
+  constexpr int NEN = ET<false>::NEN, NV = ET<false>::NV, NGP = ET<false>::NGP,
+                NT = ET<false>::NT, NST = 3 * NEN + NV;
   extern __shared__ __align__(16) unsigned char smem[];
-  SmA<HEXA>& S = *reinterpret_cast<SmA<HEXA>*>(smem);
-  Geo<HEXA, double>& G = S.G;
+  SmA& S = *reinterpret_cast<SmA*>(smem);
+  Geo<false, double>& G = S.G;
   ElemCtx& E = S.E;
   const int el = L.elems[blockIdx.x];
   if (threadIdx.x == 0) S.sFail = 0;
-  load_element<HEXA, double>(L, el, E, G);
+  load_element<false, double>(L, el, E, G);
   for (int k = threadIdx.x; k < NST; k += NT) {
     const int n = k < 3 * NEN ? E.nodes[k / 3] : E.nodes[k - 3 * NEN];
     const int q = k < 3 * NEN ? k % 3 : 3;
@@ -1103,7 +1072,7 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
   const MatConst mc = L.mat[E.mat - 1];
   double gE = 0.0, gK = 0.0, gM = 0.0;
   for (int gq = threadIdx.x; gq < NGP; gq += NT) {
-    if (!point_geometry<HEXA, double>(G, gq, nullptr)) {
+    if (!point_geometry<false, double>(G, gq, nullptr)) {
       S.sFail = 1;
       continue;
     }
@@ -1217,6 +1186,8 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
     }
   }
 }
+
+#include "pm_hexa_sum.h"
 
 // ---------------------------------------------------------------------------
 // isw = 3: stresses and Darcy fluxes at the vertices (Elmlib03.f:2206-2256
@@ -1400,6 +1371,14 @@ cudaError_t launch_elem(Kern k, int n, int nt, cudaStream_t s, Args... args) {
   return cudaGetLastError();
 }
 
+template <SfOp OP>
+cudaError_t launch_hexa_sum(const ElemLaunch& L, const double* a0, const double* a1,
+                            const double* a2, const SfLoads& ld, double* o0, double* o1,
+                            cudaStream_t s) {
+  return launch_elem<SmSf<OP>>(k_hexa_sum<OP>, L.nelem, kSfThreads, s, L, a0, a1, a2, ld, o0,
+                               o1);
+}
+
 }  // namespace
 
 cudaError_t ensure_shape_tables() {
@@ -1440,8 +1419,8 @@ cudaError_t launch_assemble_K(const ElemLaunch& L, bool hexa, double* val, cudaS
 cudaError_t launch_residual(const ElemLaunch& L, bool hexa, const double* u,
                             double* b, cudaStream_t s) {
   if (L.nelem <= 0) return cudaSuccess;
-  if (hexa) return launch_elem<SmR<true>>(k_residual<true>, L.nelem, 64, s, L, u, b);
-  return launch_elem<SmR<false>>(k_residual<false>, L.nelem, 32, s, L, u, b);
+  if (hexa) return launch_hexa_sum<kSfResidual>(L, u, nullptr, nullptr, {}, b, nullptr, s);
+  return launch_elem<SmR>(k_residual_tetra, L.nelem, 32, s, L, u, b);
 }
 
 cudaError_t launch_rhs4(const ElemLaunch& L, bool hexa, const double* u,
@@ -1450,29 +1429,10 @@ cudaError_t launch_rhs4(const ElemLaunch& L, bool hexa, const double* u,
                         const double* fload, int maxt, double* b, cudaStream_t s) {
   if (L.nelem <= 0) return cudaSuccess;
   if (hexa)
-    return launch_elem<SmF<true>>(k_rhs4<true>, L.nelem, 64, s, L, u, dp, eload, eloadp,
-                                  load, fload, maxt, b);
-  return launch_elem<SmF<false>>(k_rhs4<false>, L.nelem, 32, s, L, u, dp, eload, eloadp,
-                                 load, fload, maxt, b);
-}
-
-// (the shared-memory opt-in is set per kernel: the two modes share a
-// signature, so launch_elem's per-instantiation flag would cover only one)
-template <bool HEXA, int MODE>
-cudaError_t launch_adjoint_t(const ElemLaunch& L, const double* lam, const double* un,
-                             const double* dun, double* mu, double* nu, double* grad,
-                             cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_adjoint<HEXA, MODE>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sizeof(SmA<HEXA>));
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
-  k_adjoint<HEXA, MODE><<<L.nelem, ET<HEXA>::NT, sizeof(SmA<HEXA>), s>>>(L, lam, un, dun, mu,
-                                                                          nu, grad);
-  return cudaGetLastError();
+    return launch_hexa_sum<kSfRhs4>(L, u, dp, nullptr, {eload, eloadp, load, fload, maxt}, b,
+                                    nullptr, s);
+  return launch_elem<SmF>(k_rhs4_tetra, L.nelem, 32, s, L, u, dp, eload, eloadp, load, fload,
+                          maxt, b);
 }
 
 cudaError_t launch_adjoint(const ElemLaunch& L, bool hexa, int mode, const double* lam,
@@ -1480,10 +1440,13 @@ cudaError_t launch_adjoint(const ElemLaunch& L, bool hexa, int mode, const doubl
                            double* grad, cudaStream_t s) {
   if (L.nelem <= 0) return cudaSuccess;
   if (hexa)
-    return mode == 0 ? launch_adjoint_t<true, 0>(L, lam, un, dun, mu, nu, grad, s)
-                     : launch_adjoint_t<true, 1>(L, lam, un, dun, mu, nu, grad, s);
-  return mode == 0 ? launch_adjoint_t<false, 0>(L, lam, un, dun, mu, nu, grad, s)
-                   : launch_adjoint_t<false, 1>(L, lam, un, dun, mu, nu, grad, s);
+    return mode == 0
+               ? launch_hexa_sum<kSfApply>(L, lam, nullptr, nullptr, {}, mu, nu, s)
+               : launch_hexa_sum<kSfGrad>(L, lam, un, dun, {}, grad, nullptr, s);
+  return mode == 0
+             ? launch_elem<SmA>(k_adjoint_tetra<0>, L.nelem, 32, s, L, lam, un, dun, mu, nu, grad)
+             : launch_elem<SmA>(k_adjoint_tetra<1>, L.nelem, 32, s, L, lam, un, dun, mu, nu,
+                                grad);
 }
 
 cudaError_t launch_stress3(const ElemLaunch& L, bool hexa, const double* u,

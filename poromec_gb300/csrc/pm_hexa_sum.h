@@ -1,0 +1,454 @@
+// pm_hexa_sum.h -- the matrix-free hexa20 element passes by sum factorisation
+// (included by pm_elements.cu inside its unnamed namespace).
+//
+// What bounds them.  These passes interpolate nodal values to the 64 points and
+// sum point values back to the nodes: with 20 functions at 64 points that is
+// 11,500 FP64 multiply-adds each way per vector field, and mapping all
+// derivatives to physical coordinates 16,000 more, at 1.7 per clock and SM.  The
+// points are a 4 x 4 x 4 product, and the serendipity functions are products of
+// (1 - x) / 2, (1 + x) / 2 and 1 - x^2 of which at most one is quadratic: with the
+// corners' values and, for each mid-side node, its value less the mean of its
+// edge's ends as coefficients, one direction at a time (Orszag, "Spectral methods
+// for problems in complex geometries", J. Comput. Phys. 37, 1980) takes 3,600, and
+// only the gradients, not the functions, are mapped at a point.  The FP64 pipe is
+// still what bounds them on many elements (79 % busy), the chain of sweeps on few.
+// Less rounding too: fields enter as differences, and one mid-side term is smaller
+// than its node's value (error of isw 2's forces on a smooth field 0.7e-16 of the
+// largest against 2.3e-16 with the functions).
+//
+// One element per CTA of 192 threads: thread (point, direction) at the points,
+// one output per thread in each sweep; FP64 instructions are spread over the four
+// schedulers, since a warp's occupies one for 64 clocks.  Measured, before (every
+// function mapped, 64 threads) and now: isw 2's forces of the 40^3 cube 8.74 and
+// 2.97 ms, isw 4's 9.27 and 3.32, of the 2 x 2 x 40 column 0.43 and 0.12, 0.59 and
+// 0.28; the adjoint's two passes of the 32^3 cube 7.75 and 3.20.
+constexpr int kSfThreads = 192;
+
+// index in the 3 x 3 x 3 grid (r + 3 s + 9 t) of each node, and the corners' in
+// the 2 x 2 x 2 grid
+__constant__ int cGrid27[20] = {26, 24, 18, 20, 8, 6, 0, 2, 25, 21, 19, 23, 7, 3, 1, 5,
+                                17, 15, 9, 11};
+__constant__ int cGrid8[8] = {7, 6, 4, 5, 3, 2, 0, 1};
+
+struct SfLoads {  // isw 4 only
+  const int32_t *eload, *eloadp, *load;
+  const double* fload;
+  int maxt;
+};
+
+enum SfOp { kSfResidual, kSfRhs4, kSfApply, kSfGrad };
+
+template <SfOp OP>
+struct SmSf {
+  static constexpr bool GRAD = OP == kSfGrad, BODY = OP == kSfRhs4;
+  static constexpr int NC = GRAD ? 6 : 3;  // vector components: u, or lam and u_n
+  // linear fields: x, y, z, then the pressures the pass needs
+  static constexpr int NL = 3 + (GRAD ? 3 : OP == kSfRhs4 ? 2 : 1);
+  double C[NC][27];          // coefficients, then the sums
+  double A[2][NC][36];      // [value, derivative][c][zy x]
+  double B[NC][3][48];      // [c][r, s, t][z yx]
+  double lin[NL][8];
+  double LB[NL][48];        // d/dr (z, y), d/ds (z, x), value (z, yx)
+  double JI[3][3][64];      // [x_j][xi_a]: dx_j / dxi_a, then det dxi_a / dx_j
+  double rd[64], wq[64], w[64];  // 1 / det, the weight, weight times det
+  double G[NC][3][64];      // physical gradients, then the natural fluxes
+  double F[3][64];          // pressure flux
+  double S0[64];            // value source of the pressure rows
+  double body[BODY ? 64 : 1];
+  double T2[2][32];         // pressure rows: sweeps back
+  double LT[2][3][32];
+  double out[68], out2[8], pf[BODY ? 68 : 1];
+  double Q[4][3], Qd[4][3], Lw[4][2];
+  double gsum[3][kSfThreads / 32];
+  int nodes[20], mat;
+  int iqm[7], iqh[7], any;
+  int fail;
+};
+
+// A mid-side node's coefficient (edge e: four along r, four along s, four along
+// t), in place.
+__device__ __forceinline__ void sf_edge(double* c, int e) {
+  const int d = e >> 2, a = 2 * (e & 1), b = 2 * ((e >> 1) & 1);
+  const int sd = d == 0 ? 1 : d == 1 ? 3 : 9;
+  const int m = sd + a * (d == 0 ? 3 : 1) + b * (d == 2 ? 3 : 9);
+  c[m] -= 0.5 * (c[m - sd] + c[m + sd]);
+}
+
+// Transposed: what a node takes from the sums.
+__device__ __forceinline__ double sf_fold(const double* c, int node) {
+  const int g = cGrid27[node];
+  if (node >= 8) return c[g];
+  const int r = g % 3, s = (g / 3) % 3, t = g / 9;
+  return c[g] - 0.5 * (c[1 + 3 * s + 9 * t] + c[r + 3 + 9 * t] + c[r + 3 * s + 9]);
+}
+
+// OP kSfResidual: b -= K_e u_e (isw 2, rhs).  kSfRhs4: b -= p of isw 4 (internal
+// force of the previous state, body force, Darcy gravity term, face loads).
+// kSfApply: mu -= [Kuu lam_u ; Kpp_perm lam_p], nu -= Kpu lam_u.  kSfGrad: the
+// contractions of launch_adjoint's mode 1.  a0: u (lam for the adjoint), a1: dp
+// (u_n), a2: du.
+template <SfOp OP>
+__global__ void __launch_bounds__(kSfThreads, 5)
+    k_hexa_sum(ElemLaunch L, const double* __restrict__ a0, const double* __restrict__ a1,
+               const double* __restrict__ a2, SfLoads ld, double* __restrict__ o0,
+               double* __restrict__ o1) {
+  using Sm = SmSf<OP>;
+  constexpr int NEN = 20, NV = 8, NC = Sm::NC, NL = Sm::NL;
+  extern __shared__ __align__(16) unsigned char smem[];
+  Sm& S = *reinterpret_cast<Sm*>(smem);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int el = L.elems[blockIdx.x];
+  const int32_t* ixe = L.ix + (size_t)(NEN + 1) * (el - 1);
+  // ---- element data -----------------------------------------------------------
+  if (tid < 80) {  // vector components and pressure of node tid / 4
+    const int i = tid >> 2, q = tid & 3, n = ixe[i], n0 = ixe[0];
+    if (q < 3) {
+      // only gradients are taken of these: less node 1's value, what the sweeps
+      // round is the field's variation over the element, not the field
+      const size_t a = (size_t)kNdf * (n - 1) + q, r = (size_t)kNdf * (n0 - 1) + q;
+      S.C[q][cGrid27[i]] = a0[a] - a0[r];
+      if constexpr (Sm::GRAD) S.C[3 + q][cGrid27[i]] = a1[a] - a1[r];
+      if (i < NV) S.lin[q][cGrid8[i]] = L.x[(size_t)3 * (n - 1) + q];
+    } else {
+      S.nodes[i] = n;
+      if (i < NV) {
+        const int k = cGrid8[i];
+        S.lin[3][k] = a0[(size_t)kNdf * (n - 1) + 3];
+        if constexpr (OP == kSfRhs4) S.lin[NL - 1][k] = a1[n - 1];
+        if constexpr (Sm::GRAD) {
+          S.lin[NL - 2][k] = a1[(size_t)kNdf * (n - 1) + 3];
+          S.lin[NL - 1][k] = a2[(size_t)kNdf * (n - 1) + 3];
+        }
+      }
+    }
+  } else if (tid < 84) {  // the 1-D functions at the Gauss points
+    const int g = tid - 80;
+    const double x = cPG4[g];
+    S.Q[g][0] = 0.5 * (1.0 - x);
+    S.Q[g][1] = fma(-x, x, 1.0);
+    S.Q[g][2] = 0.5 * (1.0 + x);
+    S.Qd[g][0] = -0.5;
+    S.Qd[g][1] = -2.0 * x;
+    S.Qd[g][2] = 0.5;
+    S.Lw[g][0] = S.Q[g][0];
+    S.Lw[g][1] = S.Q[g][2];
+  } else if (tid == 84) {
+    S.mat = ixe[NEN];
+    S.fail = 0;
+    S.any = 0;
+  } else if (tid >= 128 && tid < 128 + 4 * NC) {  // no function of a face's centre
+    S.C[(tid - 128) >> 2][4 + 6 * (tid & 3)] = 0.0;
+  } else if (tid >= 96 && tid < 96 + 4 * NC) {  // nor the line through two
+    S.A[0][(tid - 96) >> 2][16 + (tid & 3)] = S.A[1][(tid - 96) >> 2][16 + (tid & 3)] = 0.0;
+  }
+  if constexpr (OP == kSfRhs4)
+    for (int k = tid - 96; k >= 0 && k < 68; k += kSfThreads) S.pf[k] = 0.0;
+  __syncthreads();
+  if (OP == kSfRhs4 && tid < 7) {
+    S.iqm[tid] = ld.eload ? ld.eload[(size_t)7 * (el - 1) + tid] : 0;
+    S.iqh[tid] = ld.eloadp ? ld.eloadp[(size_t)7 * (el - 1) + tid] : 0;
+    if (S.iqm[tid] > 0 || S.iqh[tid] > 0) S.any = 1;
+  }
+  if (tid >= 32 && tid < 32 + 12 * NC) sf_edge(S.C[(tid - 32) / 12], (tid - 32) % 12);
+  // ---- linear fields, two directions --------------------------------------------
+  for (int k = tid; k < NL * 48; k += kSfThreads) {  // (one kind per warp, or nearly)
+    const int kind = k < NL * 8 ? 0 : k < NL * 16 ? 1 : 2;
+    const int f = kind == 2 ? (k - NL * 16) >> 5 : (k - kind * NL * 8) >> 3;
+    const int o = kind == 2 ? k - NL * 16 - 32 * f : k - kind * NL * 8 - 8 * f;
+    const double* c = S.lin[f] + 4 * (kind == 2 ? o >> 4 : o >> 2);
+    const double* wx = S.Lw[o & 3];
+    if (kind == 0) {  // d/dr at (z, y)
+      S.LB[f][o] = 0.5 * ((c[1] - c[0]) * wx[0] + (c[3] - c[2]) * wx[1]);
+    } else if (kind == 1) {  // d/ds at (z, x)
+      S.LB[f][8 + o] = 0.5 * ((c[2] - c[0]) * wx[0] + (c[3] - c[1]) * wx[1]);
+    } else {  // value at (z, y, x)
+      const double* wy = S.Lw[(o >> 2) & 3];
+      S.LB[f][16 + o] =
+          (c[0] * wx[0] + c[1] * wx[1]) * wy[0] + (c[2] * wx[0] + c[3] * wx[1]) * wy[1];
+    }
+  }
+  __syncthreads();
+  // ---- vector fields: r, then s -----------------------------------------------
+  for (int k = tid; k < NC * 32; k += kSfThreads) {
+    const int c = k >> 5, l = (k >> 2) & 7, zy = l + (l > 3), x = k & 3;
+    const double* v = S.C[c] + 3 * zy;
+    S.A[0][c][zy * 4 + x] = v[0] * S.Q[x][0] + v[2] * S.Q[x][2] + v[1] * S.Q[x][1];
+    S.A[1][c][zy * 4 + x] = 0.5 * (v[2] - v[0]) + v[1] * S.Qd[x][1];
+  }
+  // the Jacobian meanwhile: thread (point, coordinate)
+  const int g = tid & 63, j = tid >> 6, yx = g & 15, zg = g >> 4;
+  const double l0 = S.Lw[zg][0], l1 = S.Lw[zg][1];
+  auto grad_lin = [&](int f, double (&n)[3]) {
+    const double* b = S.LB[f];
+    n[0] = b[yx >> 2] * l0 + b[4 + (yx >> 2)] * l1;
+    n[1] = b[8 + (yx & 3)] * l0 + b[12 + (yx & 3)] * l1;
+    n[2] = 0.5 * (b[32 + yx] - b[16 + yx]);
+  };
+  auto value_lin = [&](int f) { return S.LB[f][16 + yx] * l0 + S.LB[f][32 + yx] * l1; };
+  {
+    double n[3];
+    grad_lin(j, n);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) S.JI[j][a][g] = n[a];
+  }
+  __syncthreads();
+  for (int k = tid; k < NC * 48; k += kSfThreads) {
+    const int c = k / 48, o = k % 48, z = o >> 4, y = (o >> 2) & 3, x = o & 3;
+    double br = 0, bs = 0, bt = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double av = S.A[0][c][(3 * z + i) * 4 + x], ad = S.A[1][c][(3 * z + i) * 4 + x];
+      br += ad * S.Q[y][i];
+      bs += av * S.Qd[y][i];
+      bt += av * S.Q[y][i];
+    }
+    S.B[c][0][o] = br;
+    S.B[c][1][o] = bs;
+    S.B[c][2][o] = bt;
+  }
+  // column j of the adjugate; the first two warps also form the determinant
+  double ji[3];
+  {
+    const int j1 = j == 2 ? 0 : j + 1, j2 = j == 0 ? 2 : j - 1;
+    double m[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      m[a][0] = S.JI[j][a][g];
+      m[a][1] = S.JI[j1][a][g];
+      m[a][2] = S.JI[j2][a][g];
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const int p = (a + 1) % 3, q = (a + 2) % 3;
+      ji[a] = m[p][1] * m[q][2] - m[p][2] * m[q][1];
+    }
+    if (j == 0) {
+      const double det = m[0][0] * ji[0] + m[1][0] * ji[1] + m[2][0] * ji[2];
+      if (!(det > 1.0e-14)) S.fail = 1;
+      const double wq = cWG4[g & 3] * cWG4[(g >> 2) & 3] * cWG4[zg];
+      S.rd[g] = 1.0 / det;
+      S.wq[g] = wq;
+      S.w[g] = wq * det;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int a = 0; a < 3; ++a) S.JI[j][a][g] = ji[a];
+  // natural gradients of component j at the point
+  double h[NC / 3][3];
+#pragma unroll
+  for (int v = 0; v < NC / 3; ++v) {
+    const int c = 3 * v + j;
+    h[v][0] = h[v][1] = h[v][2] = 0.0;
+#pragma unroll
+    for (int z = 0; z < 3; ++z) {
+      h[v][0] += S.B[c][0][16 * z + yx] * S.Q[zg][z];
+      h[v][1] += S.B[c][1][16 * z + yx] * S.Q[zg][z];
+      h[v][2] += S.B[c][2][16 * z + yx] * S.Qd[zg][z];
+    }
+  }
+  __syncthreads();
+  if (S.fail) {
+    if (tid == 0) atomicOr(L.err, 1);
+    return;
+  }
+  const double rd = S.rd[g], wq = S.wq[g];
+#pragma unroll
+  for (int v = 0; v < NC / 3; ++v)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double t = h[v][0] * S.JI[k][0][g] + h[v][1] * S.JI[k][1][g] +
+                       h[v][2] * S.JI[k][2][g];
+      S.G[3 * v + j][k][g] = Sm::GRAD ? t : rd * t;  // (the contraction scales its sum)
+    }
+  // physical pressure gradient, component j
+  const MatConst mc = L.mat[S.mat - 1];
+  const double gj = j == 0 ? L.g0 : j == 1 ? L.g1 : L.g2;
+  const double dtk = mc.perm * L.dt;
+  double gp;
+  {
+    double n[3];
+    grad_lin(3, n);
+    gp = n[0] * ji[0] + n[1] * ji[1] + n[2] * ji[2];  // times det
+  }
+  // (times the weight alone: det goes into the adjugate that maps it back)
+  double gk = 0.0;
+  if constexpr (OP == kSfRhs4) {
+    S.F[j][g] = wq * dtk * (mc.fluid_d * gj - rd * gp);
+  } else if constexpr (OP != kSfGrad) {
+    S.F[j][g] = wq * dtk * (rd * gp);
+  } else {
+    double n[3];
+    grad_lin(4, n);
+    gk = wq * dtk * gp *
+         (rd * (n[0] * ji[0] + n[1] * ji[1] + n[2] * ji[2]) - mc.fluid_d * gj);
+  }
+  __syncthreads();
+  if constexpr (OP == kSfGrad) {
+    // row j of the contraction of lam's strain with u_n's stress
+    const int j1 = j == 2 ? 0 : j + 1, j2 = j == 0 ? 2 : j - 1;
+    const double s =
+        (S.G[3 + j][j][g] + mc.b * S.G[3 + j1][j1][g] + mc.b * S.G[3 + j2][j2][g]) * mc.a;
+    const double shl = S.G[j][j1][g] + S.G[j1][j][g];
+    const double shu = S.G[3 + j][j1][g] + S.G[3 + j1][j][g];
+    double v[3] = {-wq * rd * (S.G[j][j][g] * s + mc.c * mc.a * (shl * shu)), gk,
+                   j == 0 ? -S.w[g] * mc.imod_biot * value_lin(3) * value_lin(5) : 0.0};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      double x = v[k];
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+      if (lane == 0) S.gsum[k][tid >> 5] = x;
+    }
+    __syncthreads();
+    if (tid < 3) {
+      double t = 0.0;
+      for (int i = 0; i < kSfThreads / 32; ++i) t += S.gsum[tid][i];
+      o0[(size_t)3 * (el - 1) + tid] += t;
+    }
+    return;
+  } else {
+    // row j of the weight times the stress, and the sources of the pressure rows
+    double q[3];
+    {
+      const int j1 = j == 2 ? 0 : j + 1, j2 = j == 0 ? 2 : j - 1;
+      const double e0 = S.G[j][j][g], e1 = S.G[j1][j1][g], e2 = S.G[j2][j2][g];
+      double sn = (e0 + mc.b * e1 + mc.b * e2) * mc.a;
+      if constexpr (OP == kSfResidual) {
+        const double pg = value_lin(3);
+        sn -= mc.coef_biot * pg;
+        if (j == 0) S.S0[g] = S.w[g] * (mc.coef_biot * (e0 + e1 + e2) + mc.imod_biot * pg);
+      } else if constexpr (OP == kSfRhs4) {
+        sn -= mc.coef_biot * value_lin(4);
+        if (j == 0) S.body[g] = S.w[g] * mc.pm_d;
+      } else if (j == 0) {
+        S.S0[g] = S.w[g] * mc.coef_biot * (e0 + e1 + e2);
+      }
+      const double ca = mc.c * mc.a;
+      double st[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        st[k] = wq * (k == j ? sn : ca * (S.G[j][k][g] + S.G[k][j][g]));
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+        q[a] = st[0] * S.JI[0][a][g] + st[1] * S.JI[1][a][g] + st[2] * S.JI[2][a][g];
+    }
+    // natural pressure flux, component j
+    const double fa = S.F[0][g] * S.JI[0][j][g] + S.F[1][g] * S.JI[1][j][g] +
+                      S.F[2][g] * S.JI[2][j][g];
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 3; ++a) S.G[j][a][g] = q[a];
+    S.F[j][g] = fa;
+    __syncthreads();
+    // ---- back: t ----------------------------------------------------------------
+    const double gl[3] = {L.g0, L.g1, L.g2};
+    if (tid < 144) {
+      const int c = tid / 48, o = tid % 48, z = o >> 4, p = o & 15;
+      double br = 0, bs = 0, bt = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        br += S.G[c][0][16 * k + p] * S.Q[k][z];
+        bs += S.G[c][1][16 * k + p] * S.Q[k][z];
+        bt += S.G[c][2][16 * k + p] * S.Qd[k][z];
+        if constexpr (OP == kSfRhs4) bt -= S.body[16 * k + p] * gl[c] * S.Q[k][z];
+      }
+      S.B[c][0][o] = br;
+      S.B[c][1][o] = bs;
+      S.B[c][2][o] = bt;
+    } else if (tid >= 160) {  // pressure rows: (z, yx)
+      const int o = tid - 160, z = o >> 4, p = o & 15;
+      const double dz = z ? 0.5 : -0.5;
+      double tr = 0, ts = 0, tv = 0, t2 = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        tr += S.F[0][16 * k + p] * S.Lw[k][z];
+        ts += S.F[1][16 * k + p] * S.Lw[k][z];
+        tv += S.F[2][16 * k + p] * dz;
+        if (OP == kSfResidual) tv += S.S0[16 * k + p] * S.Lw[k][z];
+        if (OP == kSfApply) t2 += S.S0[16 * k + p] * S.Lw[k][z];
+      }
+      S.LT[0][0][o] = tr;
+      S.LT[0][1][o] = ts;
+      S.LT[0][2][o] = tv;
+      if (OP == kSfApply) S.LT[1][2][o] = t2;
+    }
+    __syncthreads();
+    // ---- back: s ----------------------------------------------------------------
+    if (tid < 96) {
+      const int c = tid >> 5, l = (tid >> 2) & 7, zy = l + (l > 3), x = tid & 3;
+      const int z = zy / 3, k = zy % 3;
+      double v = 0, d = 0;
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const int o = 16 * z + 4 * y + x;
+        v += S.B[c][1][o] * S.Qd[y][k] + S.B[c][2][o] * S.Q[y][k];
+        d += S.B[c][0][o] * S.Q[y][k];
+      }
+      S.A[0][c][zy * 4 + x] = v;
+      S.A[1][c][zy * 4 + x] = d;
+    } else if (tid >= 160 && tid < 176) {
+      const int o = tid - 160, z = o >> 3, k = (o >> 2) & 1, x = o & 3;
+      const double dy = k ? 0.5 : -0.5;
+      double v = 0, d = 0, v2 = 0;
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const int p = 16 * z + 4 * y + x;
+        v += S.LT[0][1][p] * dy + S.LT[0][2][p] * S.Lw[y][k];
+        d += S.LT[0][0][p] * S.Lw[y][k];
+        if (OP == kSfApply) v2 += S.LT[1][2][p] * S.Lw[y][k];
+      }
+      S.T2[0][o] = v;
+      S.T2[0][16 + o] = d;
+      if (OP == kSfApply) S.T2[1][o] = v2;
+    }
+    __syncthreads();
+    // ---- back: r ----------------------------------------------------------------
+    if (tid < 60) {
+      const int c = tid / 20, i = cGrid27[tid % 20], zy = i / 3, k = i % 3;
+      double v = 0;
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        v += S.A[0][c][zy * 4 + x] * S.Q[x][k] + S.A[1][c][zy * 4 + x] * S.Qd[x][k];
+      S.C[c][i] = v;
+    } else if (tid >= 160 && tid < 168) {
+      const int i = tid - 160, zy = i >> 1, k = i & 1;
+      const double dx = k ? 0.5 : -0.5;
+      double v = 0, v2 = 0;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        v += S.T2[0][zy * 4 + x] * S.Lw[x][k] + S.T2[0][16 + zy * 4 + x] * dx;
+        if (OP == kSfApply) v2 += S.T2[1][zy * 4 + x] * S.Lw[x][k];
+      }
+      S.out[60 + i] = v;
+      if (OP == kSfApply) S.out2[i] = v2;
+    }
+    if constexpr (OP == kSfRhs4)
+      if (S.any && tid == 128) {
+        int f = 0;
+        double xv[NV][3];
+        for (int i = 0; i < NV; ++i)
+          for (int k = 0; k < 3; ++k) xv[i][k] = S.lin[k][cGrid8[i]];
+        face_loads<true>(L, S.iqm, S.iqh, xv, ld.load, ld.fload, ld.maxt, S.pf, &f);
+        if (f) S.fail = 1;
+      }
+    __syncthreads();
+    if (OP == kSfRhs4 && S.fail) {
+      if (tid == 0) atomicOr(L.err, 1);
+      return;
+    }
+    if (tid < 60) {
+      double acc = sf_fold(S.C[tid % 3], tid / 3);
+      if constexpr (OP == kSfRhs4) acc += S.pf[tid];
+      const int e = eq_of(L, S.nodes[tid / 3], tid % 3);
+      if (e > 0) o0[e - 1] -= acc;
+    } else if (tid < 68) {
+      const int l = tid - 60, i = cGrid8[l];
+      const int e = eq_of(L, S.nodes[l], 3);
+      if (e > 0) {
+        if constexpr (OP == kSfRhs4) o0[e - 1] -= S.out[60 + i] + S.pf[tid];
+        else o0[e - 1] += S.out[60 + i];
+        if (OP == kSfApply) o1[e - 1] += S.out2[i];
+      }
+    }
+  }
+}
