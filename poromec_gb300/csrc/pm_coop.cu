@@ -534,7 +534,9 @@ cudaError_t launch(const PanelView& P, const double* val, CoopArgs A, int grid, 
   A.nloc = NPW * ((groups + grid - 1) / grid);
   const int smem = coop_local_bytes(SQMR, A.nloc);
   const void* k = SQMR ? (const void*)k_sqmr_coop<L, FUSE> : (const void*)k_pcg_coop<L, FUSE>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // the cap of every mesh, not this one's size: handles of other threads launch too
+  cudaError_t e =
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoopMaxSmem);
   if (e != cudaSuccess) return e;
   void* args[] = {(void*)&P, (void*)&val, (void*)&A};
   return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kCoopThreads), args, smem, s);
