@@ -151,6 +151,7 @@ pm::ElemLaunch elem_launch(Handle* h, int c) {
   L.elems = h->D.color_elems + h->color_ptr[c];
   L.nelem = h->color_ptr[c + 1] - h->color_ptr[c];
   L.nen = h->nen;
+  L.chain = c > 0 && h->color_ptr[c] > h->color_ptr[c - 1];
   L.node_val_off = h->P.node_val_off;
   L.node_W = h->P.node_W;
   L.dt = h->dt;

@@ -206,8 +206,8 @@ __global__ void k_fill_shape_tables() {
 
 // Integration point geometry (thread-per-point).  Returns false when the
 // determinant is <= 1e-14, the condition jacob3d_m stops on.
-template <bool HEXA, typename T>
-__device__ bool point_geometry_rst(Geo<HEXA, T>& G, int gq, T r, T s, T t, T wq, T* huv);
+template <typename T>
+__device__ bool point_geometry_tetra(Geo<false, T>& G, int gq, T r, T s, T t, T wq, T* huv);
 
 // The hexa's point geometry from the shape tables: the Jacobian from the
 // vertices, its inverse by one reciprocal of the determinant, and the
@@ -270,19 +270,18 @@ __device__ bool point_geometry(Geo<HEXA, T>& G, int gq, T* huv) {
   if constexpr (HEXA) {
     return point_geometry_hexa_tab<T>(G, gq);
   } else {
-    return point_geometry_rst<HEXA, T>(G, gq, T(cPRI4[gq]), T(cPSI4[gq]), T(cPTI4[gq]),
-                                       T(0.25), huv);
+    return point_geometry_tetra<T>(G, gq, T(cPRI4[gq]), T(cPSI4[gq]), T(cPTI4[gq]), T(0.25),
+                                   huv);
   }
 }
 
 // The geometry of point (r, s, t) with quadrature weight wq into slot gq of G
 // (slots are the integration points, or the vertices for isw 3).
-template <bool HEXA, typename T>
-__device__ bool point_geometry_rst(Geo<HEXA, T>& G, int gq, T r, T s, T t, T wq, T* huv) {
-  constexpr int NEN = ET<HEXA>::NEN, NV = ET<HEXA>::NV;
+template <typename T>
+__device__ bool point_geometry_tetra(Geo<false, T>& G, int gq, T r, T s, T t, T wq, T* huv) {
+  constexpr int NEN = ET<false>::NEN, NV = ET<false>::NV;
   T h[NV], hr[NV], hs[NV], ht[NV];
-  if (HEXA) sf_hexa8<T>(r, s, t, h, hr, hs, ht);
-  else sf_tetra4<T>(r, s, t, h, hr, hs, ht);
+  sf_tetra4<T>(r, s, t, h, hr, hs, ht);
   T J[3][3];
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
@@ -308,9 +307,8 @@ __device__ bool point_geometry_rst(Geo<HEXA, T>& G, int gq, T r, T s, T t, T wq,
   Ji[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) / det;
   Ji[1][2] = -(J[0][0] * J[1][2] - J[0][2] * J[1][0]) / det;
   Ji[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) / det;
-  T w = wq * det;
-  if (!HEXA) w = w * T(kDiv6);
-  G.w[gq] = w;
+  const T w = wq * det;
+  G.w[gq] = w * T(kDiv6);
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     G.hp[gq][k] = h[k];
@@ -319,16 +317,14 @@ __device__ bool point_geometry_rst(Geo<HEXA, T>& G, int gq, T r, T s, T t, T wq,
     G.gp[gq][k][2] = Ji[2][0] * hr[k] + Ji[2][1] * hs[k] + Ji[2][2] * ht[k];
   }
   T ur[NEN], us[NEN], ut[NEN];
-  if (HEXA) sf_hexa20_d<T>(r, s, t, ur, us, ut);
-  else sf_tetra10_d<T>(r, s, t, ur, us, ut);
+  sf_tetra10_d<T>(r, s, t, ur, us, ut);
 #pragma unroll
   for (int k = 0; k < NEN; ++k) {
     G.g[gq][k][0] = Ji[0][0] * ur[k] + Ji[0][1] * us[k] + Ji[0][2] * ut[k];
     G.g[gq][k][1] = Ji[1][0] * ur[k] + Ji[1][1] * us[k] + Ji[1][2] * ut[k];
     G.g[gq][k][2] = Ji[2][0] * ur[k] + Ji[2][1] * us[k] + Ji[2][2] * ut[k];
   }
-  if constexpr (!HEXA)
-    if (huv) sf_tetra10_v<T>(r, s, t, huv);
+  if (huv) sf_tetra10_v<T>(r, s, t, huv);
   return true;
 }
 
@@ -362,6 +358,19 @@ __device__ __forceinline__ int eq_of(const ElemLaunch& L, int n, int k) {
 // (the entry is rounded before the add: the same panels with and without RHS)
 __device__ __forceinline__ void add_val(double* val, int64_t a, double v) {
   val[a] = __dadd_rn(val[a], v);
+}
+
+// Launches of one pass, colour by colour, overlap: a colour's CTAs let the next
+// colour's start (once all of them run), and these wait before they add to what the
+// passes share (b, the panels, nodal sums), which is all that a colour writes and no
+// other input of the next.  On small meshes a launch is the latency of one element,
+// most of which comes before the adds: the 8 colours of the 2 x 2 x 40 column take
+// 116 us instead of 253 in the assembly, 32 instead of 117 in isw 2's forces.
+__device__ __forceinline__ void colour_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void colour_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 #include "pm_hexa_mma.h"
@@ -403,6 +412,7 @@ __global__ void __launch_bounds__(ET<false>::NT)
   auto& sE0 = S.sE0;
   int& sFail = S.sFail;
   const double* ul = S.ul;
+  colour_next();
   const int el = L.elems[blockIdx.x];
   if (threadIdx.x == 0) sFail = 0;
   load_element<false, double>(L, el, E, G);
@@ -426,6 +436,7 @@ __global__ void __launch_bounds__(ET<false>::NT)
   for (int gq = threadIdx.x; gq < NGP; gq += NT)
     if (!point_geometry<false, double>(G, gq, nullptr)) sFail = 1;
   __syncthreads();
+  colour_wait();
   if (sFail) {
     if (threadIdx.x == 0) atomicOr(L.err, 1);
     return;
@@ -624,6 +635,7 @@ __global__ void __launch_bounds__(ET<false>::NT)
   auto& S6 = S.S6;
   auto& Q4 = S.Q4;
   int& sFail = S.sFail;
+  colour_next();
   const int el = L.elems[blockIdx.x];
   if (threadIdx.x == 0) sFail = 0;
   load_element<false, double>(L, el, E, G);
@@ -670,6 +682,7 @@ __global__ void __launch_bounds__(ET<false>::NT)
     Q4[gq][1] = wdp * px; Q4[gq][2] = wdp * py; Q4[gq][3] = wdp * pz;
   }
   __syncthreads();
+  colour_wait();
   if (sFail) {
     if (threadIdx.x == 0) atomicOr(L.err, 1);
     return;
@@ -770,16 +783,14 @@ __device__ double d_det2(const double* hx, const double* hy, const double* xf, i
   return j00 * j11 - j10 * j01;
 }
 
-// Face tractions (types 40/41/42) and normal fluxes (43), single thread.
-template <bool HEXA>
+// Face tractions (types 40/41/42) and normal fluxes (43) of a tetra, single thread.
 __device__ void face_loads(const ElemLaunch& L, const int* iqm, const int* iqh,
                            const double xv[][3], const int32_t* load,
                            const double* fload, int maxt, double* p, int* fail) {
-  constexpr int NEN = ET<HEXA>::NEN;
-  const int nface = HEXA ? 6 : 4, nfv = HEXA ? 4 : 3, nfn = HEXA ? 8 : 6;
+  constexpr int NEN = ET<false>::NEN, nface = 4, nfv = 3, nfn = 6;
   for (int j = 1; j <= nface; ++j) {
     if (!(iqm[j - 1] > 0 || iqh[j - 1] > 0)) continue;
-    const int* fn = HEXA ? cHexaFace[j - 1] : cTetraFace[j - 1];
+    const int* fn = cTetraFace[j - 1];
     double xf[12];
     for (int i = 0; i < nfv; ++i)
       for (int k = 0; k < 3; ++k) xf[3 * i + k] = xv[fn[i] - 1][k];
@@ -787,8 +798,7 @@ __device__ void face_loads(const ElemLaunch& L, const int* iqm, const int* iqh,
     const int cargh = iqh[j - 1] != 0 ? load[3 * (iqh[j - 1] - 1)] : 0;
     double ff[3] = {0, 0, 0}, mp[3] = {0, 0, 0}, nc = 0, dd;
     if (cargm == 40 || cargm == 41 || cargm == 42) {
-      const bool normal = HEXA ? (cargm == 41) : (cargm == 41 || cargm == 42);
-      if (normal) {
+      if (cargm == 41 || cargm == 42) {
         const double v1[3] = {xf[3] - xf[0], xf[4] - xf[1], xf[5] - xf[2]};
         const double v2[3] = {xf[6] - xf[0], xf[7] - xf[1], xf[8] - xf[2]};
         ff[0] = v2[1] * v1[2] - v2[2] * v1[1];
@@ -796,8 +806,7 @@ __device__ void face_loads(const ElemLaunch& L, const int* iqm, const int* iqh,
         ff[2] = v2[0] * v1[1] - v2[1] * v1[0];
         const double tmp = 1.0 / sqrt(ff[0] * ff[0] + ff[1] * ff[1] + ff[2] * ff[2]);
         ff[0] *= tmp; ff[1] *= tmp; ff[2] *= tmp;
-        if (HEXA && j != 2) { ff[0] = -ff[0]; ff[1] = -ff[1]; ff[2] = -ff[2]; }
-        if (!HEXA && cargm == 42)
+        if (cargm == 42)
           for (int k = 0; k < 3; ++k) mp[k] = (xf[k] + xf[3 + k] + xf[6 + k]) / 3;
       }
       d_rotate_face(xf, nfv);
@@ -807,77 +816,34 @@ __device__ void face_loads(const ElemLaunch& L, const int* iqm, const int* iqh,
       } else {
         d_tload(load, fload, maxt, iqm[j - 1], L.t, mp, L.gmod, dd, ff);
       }
-      if (HEXA) {
-        for (int ly = 0; ly < 3; ++ly)
-          for (int lx = 0; lx < 3; ++lx) {
-            const double r = cPG3[lx], s = cPG3[ly];
-            const double pr = 1 + r, ps = 1 + s, mr = 1 - r, ms = 1 - s;
-            const double hx[4] = {ps * 0.25, -ps * 0.25, -ms * 0.25, ms * 0.25};
-            const double hy[4] = {pr * 0.25, mr * 0.25, -mr * 0.25, -pr * 0.25};
-            const double det = d_det2(hx, hy, xf, 4);
-            if (!(det > 1.0e-14)) *fail = 1;
-            const double w = cWG3[lx] * cWG3[ly] * det;
-            double h[8];
-            const double mrr = 1 - r * r, mss = 1 - s * s;
-            h[4] = mrr * ps * 0.5; h[5] = mss * mr * 0.5; h[6] = mrr * ms * 0.5;
-            h[7] = mss * pr * 0.5;
-            h[0] = pr * ps * 0.25 - h[4] * 0.5 - h[7] * 0.5;
-            h[1] = mr * ps * 0.25 - h[4] * 0.5 - h[5] * 0.5;
-            h[2] = mr * ms * 0.25 - h[5] * 0.5 - h[6] * 0.5;
-            h[3] = pr * ms * 0.25 - h[6] * 0.5 - h[7] * 0.5;
-            for (int i = 0; i < nfn; ++i) {
-              const int no = fn[i];
-              const double wt1 = h[i] * w;
-              p[3 * no - 3] -= ff[0] * wt1;
-              p[3 * no - 2] -= ff[1] * wt1;
-              p[3 * no - 1] -= ff[2] * wt1;
-            }
-          }
-      } else {
-        for (int lx = 0; lx < 3; ++lx) {
-          const double r = cPRI2[lx], s = cPSI2[lx], t = 1 - r - s;
-          const double hx[3] = {1, 0, -1}, hy[3] = {0, 1, -1};
-          const double det = d_det2(hx, hy, xf, 3);
-          if (!(det > 1.0e-14)) *fail = 1;
-          const double w = 0.5 * (cWF2 * det);
-          const double h[6] = {r * (2 * r - 1), s * (2 * s - 1), t * (2 * t - 1),
-                               4 * r * s, 4 * s * t, 4 * t * r};
-          for (int i = 0; i < nfn; ++i) {
-            const int no = fn[i];
-            const double wt1 = h[i] * w;
-            p[3 * no - 3] -= ff[0] * wt1;
-            p[3 * no - 2] -= ff[1] * wt1;
-            p[3 * no - 1] -= ff[2] * wt1;
-          }
+      for (int lx = 0; lx < 3; ++lx) {
+        const double r = cPRI2[lx], s = cPSI2[lx], t = 1 - r - s;
+        const double hx[3] = {1, 0, -1}, hy[3] = {0, 1, -1};
+        const double det = d_det2(hx, hy, xf, 3);
+        if (!(det > 1.0e-14)) *fail = 1;
+        const double w = 0.5 * (cWF2 * det);
+        const double h[6] = {r * (2 * r - 1), s * (2 * s - 1), t * (2 * t - 1),
+                             4 * r * s, 4 * s * t, 4 * t * r};
+        for (int i = 0; i < nfn; ++i) {
+          const int no = fn[i];
+          const double wt1 = h[i] * w;
+          p[3 * no - 3] -= ff[0] * wt1;
+          p[3 * no - 2] -= ff[1] * wt1;
+          p[3 * no - 1] -= ff[2] * wt1;
         }
       }
     }
     if (cargh == 43) {
       d_rotate_face(xf, nfv);
       d_tload(load, fload, maxt, iqh[j - 1], L.t, mp, L.gmod, nc, &dd);
-      if (HEXA) {
-        for (int ly = 0; ly < 3; ++ly)
-          for (int lx = 0; lx < 3; ++lx) {
-            const double r = cPG3[lx], s = cPG3[ly];
-            const double pr = 1 + r, ps = 1 + s, mr = 1 - r, ms = 1 - s;
-            const double hx[4] = {ps * 0.25, -ps * 0.25, -ms * 0.25, ms * 0.25};
-            const double hy[4] = {pr * 0.25, mr * 0.25, -mr * 0.25, -pr * 0.25};
-            const double h[4] = {pr * ps * 0.25, mr * ps * 0.25, mr * ms * 0.25, pr * ms * 0.25};
-            const double det = d_det2(hx, hy, xf, 4);
-            if (!(det > 1.0e-14)) *fail = 1;
-            const double w = cWG3[lx] * cWG3[ly] * det * L.dt * nc;
-            for (int i = 0; i < 4; ++i) p[3 * NEN + fn[i] - 1] -= h[i] * w;
-          }
-      } else {
-        for (int lx = 0; lx < 3; ++lx) {
-          const double r = cPRI2[lx], s = cPSI2[lx];
-          const double hx[3] = {1, 0, -1}, hy[3] = {0, 1, -1};
-          const double h[3] = {r, s, 1 - r - s};
-          const double det = d_det2(hx, hy, xf, 3);
-          if (!(det > 1.0e-14)) *fail = 1;
-          const double w = 0.5 * (cWF2 * det) * L.dt * nc;
-          for (int i = 0; i < 3; ++i) p[3 * NEN + fn[i] - 1] -= h[i] * w;
-        }
+      for (int lx = 0; lx < 3; ++lx) {
+        const double r = cPRI2[lx], s = cPSI2[lx];
+        const double hx[3] = {1, 0, -1}, hy[3] = {0, 1, -1};
+        const double h[3] = {r, s, 1 - r - s};
+        const double det = d_det2(hx, hy, xf, 3);
+        if (!(det > 1.0e-14)) *fail = 1;
+        const double w = 0.5 * (cWF2 * det) * L.dt * nc;
+        for (int i = 0; i < 3; ++i) p[3 * NEN + fn[i] - 1] -= h[i] * w;
       }
     }
   }
@@ -917,6 +883,7 @@ __global__ void __launch_bounds__(ET<false>::NT)
   auto& iqh = S.iqh;
   int& sFail = S.sFail;
   int& sAny = S.sAny;
+  colour_next();
   const int el = L.elems[blockIdx.x];
   if (threadIdx.x == 0) { sFail = 0; sAny = 0; }
   load_element<false, double>(L, el, E, G);
@@ -978,10 +945,11 @@ __global__ void __launch_bounds__(ET<false>::NT)
   __syncthreads();
   if (sAny && threadIdx.x == 0) {
     int f = 0;
-    face_loads<false>(L, iqm, iqh, G.xv, load, fload, maxt, pf, &f);
+    face_loads(L, iqm, iqh, G.xv, load, fload, maxt, pf, &f);
     if (f) sFail = 1;
   }
   __syncthreads();
+  colour_wait();
   if (sFail) {
     if (threadIdx.x == 0) atomicOr(L.err, 1);
     return;
@@ -1057,6 +1025,7 @@ __global__ void __launch_bounds__(ET<false>::NT)
   SmA& S = *reinterpret_cast<SmA*>(smem);
   Geo<false, double>& G = S.G;
   ElemCtx& E = S.E;
+  colour_next();
   const int el = L.elems[blockIdx.x];
   if (threadIdx.x == 0) S.sFail = 0;
   load_element<false, double>(L, el, E, G);
@@ -1135,6 +1104,7 @@ __global__ void __launch_bounds__(ET<false>::NT)
     }
   }
   __syncthreads();
+  colour_wait();
   if (S.sFail) {
     if (threadIdx.x == 0) atomicOr(L.err, 1);
     return;
@@ -1195,40 +1165,38 @@ __global__ void __launch_bounds__(ET<false>::NT)
 // average (Pform.f:433-640).  At vertex i (natural coordinates of the
 // element's vertex table): total stress D eps(u) - alpha dp_i, Biot stress
 // total + alpha p_i (normal components), flux perm (rho_f g - grad p) with
-// the linear pressure gradient.  One thread per vertex; one colour per
-// launch, so no two elements of a launch share a vertex.  MODE 7 is the
+// the linear pressure gradient.  Here tetra10, one thread per vertex (hexa20:
+// k_hexa_vertex); one colour per launch, so no two elements of a launch share
+// a vertex.  MODE 7 is the
 // porosity change of porosity_form (Pform.f:969-1175; Elmlib03.f:2605-2631):
 // alpha tr(eps(du)) + dp_i / M at vertex i, with u the step's increments.
 // ---------------------------------------------------------------------------
-__constant__ double cRNH[8] = {1, -1, -1, 1, 1, -1, -1, 1};
-__constant__ double cSNH[8] = {1, 1, -1, -1, 1, 1, -1, -1};
-__constant__ double cTNH[8] = {1, 1, 1, 1, -1, -1, -1, -1};
 __constant__ double cRNT[4] = {1, 0, 0, 0};
 __constant__ double cSNT[4] = {0, 1, 0, 0};
 __constant__ double cTNT[4] = {0, 0, 1, 0};
 
-template <bool HEXA>
 struct Sm3 {
-  Geo<HEXA, double> G;
-  double ul[3 * ET<HEXA>::NEN + ET<HEXA>::NV];
-  double dpl[ET<HEXA>::NV];
+  Geo<false, double> G;
+  double ul[3 * ET<false>::NEN + ET<false>::NV];
+  double dpl[ET<false>::NV];
   ElemCtx E;
   int sFail;
 };
 
-template <bool HEXA, int MODE>
-__global__ void __launch_bounds__(ET<HEXA>::NT)
-    k_vertex(ElemLaunch L, const double* __restrict__ u, const double* __restrict__ dp,
+template <int MODE>
+__global__ void __launch_bounds__(ET<false>::NT)
+    k_vertex_tetra(ElemLaunch L, const double* __restrict__ u, const double* __restrict__ dp,
              double* __restrict__ tx, double* __restrict__ txb, double* __restrict__ flux) {
-  constexpr int NEN = ET<HEXA>::NEN, NV = ET<HEXA>::NV, NT = ET<HEXA>::NT,
+  constexpr int NEN = ET<false>::NEN, NV = ET<false>::NV, NT = ET<false>::NT,
                 NST = 3 * NEN + NV;
   extern __shared__ __align__(16) unsigned char smem[];
-  Sm3<HEXA>& S = *reinterpret_cast<Sm3<HEXA>*>(smem);
-  Geo<HEXA, double>& G = S.G;
+  Sm3& S = *reinterpret_cast<Sm3*>(smem);
+  Geo<false, double>& G = S.G;
   ElemCtx& E = S.E;
+  colour_next();
   const int el = L.elems[blockIdx.x];
   if (threadIdx.x == 0) S.sFail = 0;
-  load_element<HEXA, double>(L, el, E, G);
+  load_element<false, double>(L, el, E, G);
   for (int k = threadIdx.x; k < NST; k += NT) {
     const int n = k < 3 * NEN ? E.nodes[k / 3] : E.nodes[k - 3 * NEN];
     const int q = k < 3 * NEN ? k % 3 : 3;
@@ -1239,11 +1207,11 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
   __syncthreads();
   const int i = threadIdx.x;
   if (i < NV) {
-    const double r = HEXA ? cRNH[i] : cRNT[i], sv = HEXA ? cSNH[i] : cSNT[i],
-                 tv = HEXA ? cTNH[i] : cTNT[i];
-    if (!point_geometry_rst<HEXA, double>(G, i, r, sv, tv, 1.0, nullptr)) S.sFail = 1;
+    if (!point_geometry_tetra<double>(G, i, cRNT[i], cSNT[i], cTNT[i], 1.0, nullptr))
+      S.sFail = 1;
   }
   __syncthreads();
+  colour_wait();
   if (S.sFail) {
     if (threadIdx.x == 0) atomicOr(L.err, 1);
     return;
@@ -1349,8 +1317,10 @@ __global__ void __launch_bounds__(ET<HEXA>::NT)
 
 // Launch helper: dynamic shared memory sized by the kernel's struct, with the
 // opt-in above 48 KB set once per kernel.
+// chain: the stream's last launch is of the same pass, so this one may start beside it
+// (the kernel calls colour_next and colour_wait).
 template <typename Sm, typename Kern, typename... Args>
-cudaError_t launch_elem(Kern k, int n, int nt, cudaStream_t s, Args... args) {
+cudaError_t launch_elem(Kern k, bool chain, int n, int nt, cudaStream_t s, Args... args) {
   // kernels of one signature and shared-memory struct (an assembly with and
   // without the fused product) share this instantiation: key on the kernel
   static std::mutex mu;
@@ -1367,16 +1337,28 @@ cudaError_t launch_elem(Kern k, int n, int nt, cudaStream_t s, Args... args) {
       opted.push_back(key);
     }
   }
-  k<<<n, nt, sizeof(Sm), s>>>(args...);
-  return cudaGetLastError();
+  // a captured launch keeps its full dependency
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (chain && (e = cudaStreamIsCapturing(s, &cap)) != cudaSuccess) return e;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)n);
+  cfg.blockDim = dim3((unsigned)nt);
+  cfg.dynamicSmemBytes = sizeof(Sm);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = chain && cap == cudaStreamCaptureStatusNone ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
 template <SfOp OP>
 cudaError_t launch_hexa_sum(const ElemLaunch& L, const double* a0, const double* a1,
                             const double* a2, const SfLoads& ld, double* o0, double* o1,
                             cudaStream_t s) {
-  return launch_elem<SmSf<OP>>(k_hexa_sum<OP>, L.nelem, kSfThreads, s, L, a0, a1, a2, ld, o0,
-                               o1);
+  return launch_elem<SmSf<OP>>(k_hexa_sum<OP>, L.chain, L.nelem, kSfThreads, s, L, a0, a1, a2,
+                               ld, o0, o1);
 }
 
 }  // namespace
@@ -1406,21 +1388,23 @@ cudaError_t launch_assemble_K(const ElemLaunch& L, bool hexa, double* val, cudaS
   if (L.nelem <= 0) return cudaSuccess;
   if (b) {
     if (hexa)
-      return launch_elem<SmHx>(k_assemble_hexa<true>, L.nelem, kHxThreads, s, L, val, u, b);
-    return launch_elem<SmK>(k_assemble_tetra<true>, L.nelem, 32, s, L, val, u, b);
+      return launch_elem<SmHx>(k_assemble_hexa<true>, L.chain, L.nelem, kHxThreads, s, L, val,
+                               u, b);
+    return launch_elem<SmK>(k_assemble_tetra<true>, L.chain, L.nelem, 32, s, L, val, u, b);
   }
   const double* nu = nullptr;
   double* nb = nullptr;
   if (hexa)
-    return launch_elem<SmHx>(k_assemble_hexa<false>, L.nelem, kHxThreads, s, L, val, nu, nb);
-  return launch_elem<SmK>(k_assemble_tetra<false>, L.nelem, 32, s, L, val, nu, nb);
+    return launch_elem<SmHx>(k_assemble_hexa<false>, L.chain, L.nelem, kHxThreads, s, L, val, nu,
+                             nb);
+  return launch_elem<SmK>(k_assemble_tetra<false>, L.chain, L.nelem, 32, s, L, val, nu, nb);
 }
 
 cudaError_t launch_residual(const ElemLaunch& L, bool hexa, const double* u,
                             double* b, cudaStream_t s) {
   if (L.nelem <= 0) return cudaSuccess;
   if (hexa) return launch_hexa_sum<kSfResidual>(L, u, nullptr, nullptr, {}, b, nullptr, s);
-  return launch_elem<SmR>(k_residual_tetra, L.nelem, 32, s, L, u, b);
+  return launch_elem<SmR>(k_residual_tetra, L.chain, L.nelem, 32, s, L, u, b);
 }
 
 cudaError_t launch_rhs4(const ElemLaunch& L, bool hexa, const double* u,
@@ -1431,8 +1415,8 @@ cudaError_t launch_rhs4(const ElemLaunch& L, bool hexa, const double* u,
   if (hexa)
     return launch_hexa_sum<kSfRhs4>(L, u, dp, nullptr, {eload, eloadp, load, fload, maxt}, b,
                                     nullptr, s);
-  return launch_elem<SmF>(k_rhs4_tetra, L.nelem, 32, s, L, u, dp, eload, eloadp, load, fload,
-                          maxt, b);
+  return launch_elem<SmF>(k_rhs4_tetra, L.chain, L.nelem, 32, s, L, u, dp, eload, eloadp, load,
+                          fload, maxt, b);
 }
 
 cudaError_t launch_adjoint(const ElemLaunch& L, bool hexa, int mode, const double* lam,
@@ -1444,9 +1428,10 @@ cudaError_t launch_adjoint(const ElemLaunch& L, bool hexa, int mode, const doubl
                ? launch_hexa_sum<kSfApply>(L, lam, nullptr, nullptr, {}, mu, nu, s)
                : launch_hexa_sum<kSfGrad>(L, lam, un, dun, {}, grad, nullptr, s);
   return mode == 0
-             ? launch_elem<SmA>(k_adjoint_tetra<0>, L.nelem, 32, s, L, lam, un, dun, mu, nu, grad)
-             : launch_elem<SmA>(k_adjoint_tetra<1>, L.nelem, 32, s, L, lam, un, dun, mu, nu,
-                                grad);
+             ? launch_elem<SmA>(k_adjoint_tetra<0>, L.chain, L.nelem, 32, s, L, lam, un, dun, mu,
+                                nu, grad)
+             : launch_elem<SmA>(k_adjoint_tetra<1>, L.chain, L.nelem, 32, s, L, lam, un, dun, mu,
+                                nu, grad);
 }
 
 cudaError_t launch_stress3(const ElemLaunch& L, bool hexa, const double* u,
@@ -1454,27 +1439,27 @@ cudaError_t launch_stress3(const ElemLaunch& L, bool hexa, const double* u,
                            cudaStream_t s) {
   if (L.nelem <= 0) return cudaSuccess;
   if (hexa)
-    return launch_elem<Sm3<true>>(k_vertex<true, 3>, L.nelem, 64, s, L, u, dp, tx, txb, flux);
-  return launch_elem<Sm3<false>>(k_vertex<false, 3>, L.nelem, 32, s, L, u, dp, tx, txb, flux);
+    return launch_elem<SmHvs>(k_hexa_vertex<3>, L.chain, (L.nelem + kHvWarps - 1) / kHvWarps,
+                              32 * kHvWarps, s, L, u, dp, tx, txb, flux);
+  return launch_elem<Sm3>(k_vertex_tetra<3>, L.chain, L.nelem, 32, s, L, u, dp, tx, txb, flux);
 }
 
 cudaError_t launch_poro7(const ElemLaunch& L, bool hexa, const double* du, double* dporo,
                          cudaStream_t s) {
   if (L.nelem <= 0) return cudaSuccess;
   if (hexa)
-    return launch_elem<Sm3<true>>(k_vertex<true, 7>, L.nelem, 64, s, L, du,
-                                  (const double*)nullptr, dporo, (double*)nullptr,
-                                  (double*)nullptr);
-  return launch_elem<Sm3<false>>(k_vertex<false, 7>, L.nelem, 32, s, L, du,
-                                 (const double*)nullptr, dporo, (double*)nullptr,
-                                 (double*)nullptr);
+    return launch_elem<SmHvs>(k_hexa_vertex<7>, L.chain, (L.nelem + kHvWarps - 1) / kHvWarps,
+                              32 * kHvWarps, s, L, du, (const double*)nullptr, dporo,
+                              (double*)nullptr, (double*)nullptr);
+  return launch_elem<Sm3>(k_vertex_tetra<7>, L.chain, L.nelem, 32, s, L, du,
+                          (const double*)nullptr, dporo, (double*)nullptr, (double*)nullptr);
 }
 
 cudaError_t launch_stress5(const ElemLaunch& L, bool hexa, const double* tx0,
                            double* b, cudaStream_t s) {
   if (L.nelem <= 0) return cudaSuccess;
-  if (hexa) return launch_elem<Sm5<true>>(k_stress5<true>, L.nelem, 64, s, L, tx0, b);
-  return launch_elem<Sm5<false>>(k_stress5<false>, L.nelem, 32, s, L, tx0, b);
+  if (hexa) return launch_elem<Sm5<true>>(k_stress5<true>, false, L.nelem, 64, s, L, tx0, b);
+  return launch_elem<Sm5<false>>(k_stress5<false>, false, L.nelem, 32, s, L, tx0, b);
 }
 
 }  // namespace pm

@@ -176,6 +176,7 @@ __global__ void __launch_bounds__(kHxThreads, 2)
   extern __shared__ __align__(16) unsigned char smem[];
   SmHx& S = *reinterpret_cast<SmHx*>(smem);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  colour_next();
   const int el = L.elems[blockIdx.x];
   const int32_t* ixe = L.ix + (size_t)(NEN + 1) * (el - 1);
   // ---- element data ---------------------------------------------------------
@@ -258,6 +259,7 @@ __global__ void __launch_bounds__(kHxThreads, 2)
   __syncthreads();
   if (S.fail) {
     if (tid == 0) atomicOr(L.err, 1);
+    colour_wait();
     return;
   }
   {
@@ -356,6 +358,7 @@ __global__ void __launch_bounds__(kHxThreads, 2)
     }
   }
   __syncthreads();
+  colour_wait();
   // ---- blocks of the element matrix ---------------------------------------------
   const MatConst mc = L.mat[S.mat - 1];
   const int32_t* slot = L.slot + (size_t)NEN * NEN * blockIdx.x;

@@ -20,8 +20,8 @@
 // one output per thread in each sweep; FP64 instructions are spread over the four
 // schedulers, since a warp's occupies one for 64 clocks.  Measured, before (every
 // function mapped, 64 threads) and now: isw 2's forces of the 40^3 cube 8.74 and
-// 2.97 ms, isw 4's 9.27 and 3.32, of the 2 x 2 x 40 column 0.43 and 0.12, 0.59 and
-// 0.28; the adjoint's two passes of the 32^3 cube 7.75 and 3.20.
+// 2.91 ms, isw 4's 9.27 and 3.11, of the 2 x 2 x 40 column 0.43 and 0.03, 0.59 and
+// 0.05 (colours overlapped); the adjoint's two passes of the 32^3 cube 7.75 and 3.12.
 constexpr int kSfThreads = 192;
 
 // index in the 3 x 3 x 3 grid (r + 3 s + 9 t) of each node, and the corners' in
@@ -82,6 +82,135 @@ __device__ __forceinline__ double sf_fold(const double* c, int node) {
   return c[g] - 0.5 * (c[1 + 3 * s + 9 * t] + c[r + 3 + 9 * t] + c[r + 3 * s + 9]);
 }
 
+// Face tractions (types 40, 41) and normal fluxes (43) of one element by one warp,
+// into p: what does not depend on the point on every lane alike, a division of the
+// rotation and a point of the 3 x 3 rule per lane, then an entry of p per lane over
+// the points in order.  wt: 72 doubles of scratch.  One thread took 42 us of a launch.
+__device__ bool hexa_face_loads(const ElemLaunch& L, const SfLoads& ld, const int* iqm,
+                                const int* iqh, const double (*lin)[8], double* p, double* wt,
+                                int lane) {
+  bool fail = false;
+  // (rotated in place a second time where a face has both loads, as the reference)
+  auto rotate = [lane](double (&xf)[12]) {
+    const double v1x = xf[3] - xf[0], v1y = xf[4] - xf[1], v1z = xf[5] - xf[2];
+    double v2x = xf[6] - xf[0], v2y = xf[7] - xf[1], v2z = xf[8] - xf[2];
+    const double v3x = v1y * v2z - v1z * v2y, v3y = v1z * v2x - v1x * v2z,
+                 v3z = v1x * v2y - v1y * v2x;
+    v2x = v1z * v3y - v1y * v3z;
+    v2y = v1x * v3z - v1z * v3x;
+    v2z = v1y * v3x - v1x * v3y;
+    const int r = lane < 3 ? 0 : lane < 6 ? 1 : 2, c = lane - 3 * r;
+    const double x = r == 0 ? v1x : r == 1 ? v2x : v3x, y = r == 0 ? v1y : r == 1 ? v2y : v3y,
+                 z = r == 0 ? v1z : r == 1 ? v2z : v3z;
+    const double n = sqrt(x * x + y * y + z * z);
+    const double q = (c == 0 ? x : c == 1 ? y : z) / n;
+    double R[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) R[k] = __shfl_sync(0xffffffffu, q, k);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      double* v = xf + 3 * i;
+      const double a = R[0] * v[0] + R[1] * v[1] + R[2] * v[2];
+      const double b = R[3] * v[0] + R[4] * v[1] + R[5] * v[2];
+      const double d = R[6] * v[0] + R[7] * v[1] + R[8] * v[2];
+      v[0] = a;
+      v[1] = b;
+      v[2] = d;
+    }
+  };
+  const int ly = lane / 3, lx = lane - 3 * ly;
+  // the point's weight times its determinant
+  auto point = [&](const double (&xf)[12], double& r, double& s) {
+    r = cPG3[lx];
+    s = cPG3[ly];
+    const double pr = 1 + r, ps = 1 + s, mr = 1 - r, ms = 1 - s;
+    const double hx[4] = {ps * 0.25, -ps * 0.25, -ms * 0.25, ms * 0.25};
+    const double hy[4] = {pr * 0.25, mr * 0.25, -mr * 0.25, -pr * 0.25};
+    const double det = d_det2(hx, hy, xf, 4);
+    if (!(det > 1.0e-14)) fail = true;
+    return cWG3[lx] * cWG3[ly] * det;
+  };
+  for (int j = 0; j < 6; ++j) {
+    if (!(iqm[j] > 0 || iqh[j] > 0)) continue;
+    const int* fn = cHexaFace[j];
+    double xf[12];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) xf[3 * i + k] = lin[k][cGrid8[fn[i] - 1]];
+    const int cargm = iqm[j] != 0 ? ld.load[3 * (iqm[j] - 1)] : 0;
+    const int cargh = iqh[j] != 0 ? ld.load[3 * (iqh[j] - 1)] : 0;
+    double ff[3] = {0, 0, 0}, nc = 0, dd;
+    const double mp[3] = {0, 0, 0};
+    if (cargm == 40 || cargm == 41 || cargm == 42) {
+      if (cargm == 41) {
+        const double v1[3] = {xf[3] - xf[0], xf[4] - xf[1], xf[5] - xf[2]};
+        const double v2[3] = {xf[6] - xf[0], xf[7] - xf[1], xf[8] - xf[2]};
+        ff[0] = v2[1] * v1[2] - v2[2] * v1[1];
+        ff[1] = v2[2] * v1[0] - v2[0] * v1[2];
+        ff[2] = v2[0] * v1[1] - v2[1] * v1[0];
+        const double tmp = 1.0 / sqrt(ff[0] * ff[0] + ff[1] * ff[1] + ff[2] * ff[2]);
+        ff[0] *= tmp; ff[1] *= tmp; ff[2] *= tmp;
+        if (j != 1) { ff[0] = -ff[0]; ff[1] = -ff[1]; ff[2] = -ff[2]; }
+      }
+      rotate(xf);
+      if (cargm == 41 || cargm == 42) {
+        d_tload(ld.load, ld.fload, ld.maxt, iqm[j], L.t, mp, L.gmod, nc, &dd);
+        ff[0] *= nc; ff[1] *= nc; ff[2] *= nc;
+      } else {
+        d_tload(ld.load, ld.fload, ld.maxt, iqm[j], L.t, mp, L.gmod, dd, ff);
+      }
+      if (lane < 9) {
+        double r, s;
+        const double w = point(xf, r, s);
+        const double pr = 1 + r, ps = 1 + s, mr = 1 - r, ms = 1 - s;
+        double h[8];
+        const double mrr = 1 - r * r, mss = 1 - s * s;
+        h[4] = mrr * ps * 0.5; h[5] = mss * mr * 0.5; h[6] = mrr * ms * 0.5;
+        h[7] = mss * pr * 0.5;
+        h[0] = pr * ps * 0.25 - h[4] * 0.5 - h[7] * 0.5;
+        h[1] = mr * ps * 0.25 - h[4] * 0.5 - h[5] * 0.5;
+        h[2] = mr * ms * 0.25 - h[5] * 0.5 - h[6] * 0.5;
+        h[3] = pr * ms * 0.25 - h[6] * 0.5 - h[7] * 0.5;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) wt[8 * lane + i] = h[i] * w;
+      }
+      __syncwarp();
+      if (lane < 24) {
+        const int i = lane / 3, k = lane - 3 * i, e = 3 * fn[i] - 3 + k;
+        const double f = k == 0 ? ff[0] : k == 1 ? ff[1] : ff[2];
+        double acc = p[e];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) acc -= f * wt[8 * q + i];
+        p[e] = acc;
+      }
+      __syncwarp();
+    }
+    if (cargh == 43) {
+      rotate(xf);
+      d_tload(ld.load, ld.fload, ld.maxt, iqh[j], L.t, mp, L.gmod, nc, &dd);
+      if (lane < 9) {
+        double r, s;
+        const double w = point(xf, r, s) * L.dt * nc;
+        const double pr = 1 + r, ps = 1 + s, mr = 1 - r, ms = 1 - s;
+        const double h[4] = {pr * ps * 0.25, mr * ps * 0.25, mr * ms * 0.25, pr * ms * 0.25};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) wt[8 * lane + i] = h[i] * w;
+      }
+      __syncwarp();
+      if (lane < 4) {
+        const int e = 60 + fn[lane] - 1;
+        double acc = p[e];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) acc -= wt[8 * q + lane];
+        p[e] = acc;
+      }
+      __syncwarp();
+    }
+  }
+  return __any_sync(0xffffffffu, fail);
+}
+
 // OP kSfResidual: b -= K_e u_e (isw 2, rhs).  kSfRhs4: b -= p of isw 4 (internal
 // force of the previous state, body force, Darcy gravity term, face loads).
 // kSfApply: mu -= [Kuu lam_u ; Kpp_perm lam_p], nu -= Kpu lam_u.  kSfGrad: the
@@ -97,6 +226,7 @@ __global__ void __launch_bounds__(kSfThreads, 5)
   extern __shared__ __align__(16) unsigned char smem[];
   Sm& S = *reinterpret_cast<Sm*>(smem);
   const int tid = threadIdx.x, lane = tid & 31;
+  colour_next();
   const int el = L.elems[blockIdx.x];
   const int32_t* ixe = L.ix + (size_t)(NEN + 1) * (el - 1);
   // ---- element data -----------------------------------------------------------
@@ -250,6 +380,7 @@ __global__ void __launch_bounds__(kSfThreads, 5)
   __syncthreads();
   if (S.fail) {
     if (tid == 0) atomicOr(L.err, 1);
+    colour_wait();
     return;
   }
   const double rd = S.rd[g], wq = S.wq[g];
@@ -300,6 +431,7 @@ __global__ void __launch_bounds__(kSfThreads, 5)
       if (lane == 0) S.gsum[k][tid >> 5] = x;
     }
     __syncthreads();
+    colour_wait();
     if (tid < 3) {
       double t = 0.0;
       for (int i = 0; i < kSfThreads / 32; ++i) t += S.gsum[tid][i];
@@ -374,6 +506,12 @@ __global__ void __launch_bounds__(kSfThreads, 5)
     }
     __syncthreads();
     // ---- back: s ----------------------------------------------------------------
+    if constexpr (OP == kSfRhs4)
+      if (S.any && tid >= 128 && tid < 160) {  // (G is read)
+        if (hexa_face_loads(L, ld, S.iqm, S.iqh, S.lin, S.pf, &S.G[0][0][0], lane) &&
+            lane == 0)
+          S.fail = 1;
+      }
     if (tid < 96) {
       const int c = tid >> 5, l = (tid >> 2) & 7, zy = l + (l > 3), x = tid & 3;
       const int z = zy / 3, k = zy % 3;
@@ -422,16 +560,8 @@ __global__ void __launch_bounds__(kSfThreads, 5)
       S.out[60 + i] = v;
       if (OP == kSfApply) S.out2[i] = v2;
     }
-    if constexpr (OP == kSfRhs4)
-      if (S.any && tid == 128) {
-        int f = 0;
-        double xv[NV][3];
-        for (int i = 0; i < NV; ++i)
-          for (int k = 0; k < 3; ++k) xv[i][k] = S.lin[k][cGrid8[i]];
-        face_loads<true>(L, S.iqm, S.iqh, xv, ld.load, ld.fload, ld.maxt, S.pf, &f);
-        if (f) S.fail = 1;
-      }
     __syncthreads();
+    colour_wait();
     if (OP == kSfRhs4 && S.fail) {
       if (tid == 0) atomicOr(L.err, 1);
       return;
@@ -449,6 +579,114 @@ __global__ void __launch_bounds__(kSfThreads, 5)
         else o0[e - 1] += S.out[60 + i];
         if (OP == kSfApply) o1[e - 1] += S.out2[i];
       }
+    }
+  }
+}
+
+// isw 3 (MODE 3) and the porosity change (MODE 7) at the 8 vertices (see k_vertex_tetra):
+// there the derivative along a direction is that of the edge's three nodes, and the
+// Jacobian's row half the edge.  A warp per element, thread (vertex, coordinate); the
+// latency of one element bounds it.  The 20 functions' derivatives by a thread per
+// vertex took 33 us a launch on the 2 x 2 x 40 column.
+constexpr int kHvWarps = 4;
+struct SmHv {
+  double c[3][27];  // displacements on the 3 x 3 x 3 grid
+  double l[4][8];   // coordinates, pressure
+  double J[3][3][8];
+  double G[3][3][8];
+};
+struct SmHvs {
+  SmHv warp[kHvWarps];
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(32 * kHvWarps)
+    k_hexa_vertex(ElemLaunch L, const double* __restrict__ u, const double* __restrict__ dp,
+                  double* __restrict__ tx, double* __restrict__ txb,
+                  double* __restrict__ flux) {
+  constexpr int NEN = 20;
+  extern __shared__ __align__(16) unsigned char smem[];
+  SmHv& S = reinterpret_cast<SmHvs*>(smem)->warp[threadIdx.x >> 5];
+  colour_next();
+  const int lane = threadIdx.x & 31;
+  const int ie = blockIdx.x * kHvWarps + (threadIdx.x >> 5);
+  if (ie >= L.nelem) {
+    colour_wait();
+    return;
+  }
+  const int32_t* ixe = L.ix + (size_t)(NEN + 1) * (L.elems[ie] - 1);
+  for (int k = lane; k < 3 * NEN; k += 32)
+    S.c[k % 3][cGrid27[k / 3]] = u[(size_t)kNdf * (ixe[k / 3] - 1) + k % 3];
+  {
+    const int n = ixe[lane >> 2] - 1, q = lane & 3;
+    S.l[q][cGrid8[lane >> 2]] = q < 3 ? L.x[(size_t)3 * n + q] : u[(size_t)kNdf * n + 3];
+  }
+  const MatConst mc = L.mat[ixe[NEN] - 1];
+  __syncwarp();
+  // vertex i at corner g of the grid (bit a: side of direction a), coordinate j;
+  // lanes 24..31 repeat coordinate 2
+  const int i = lane & 7, j = min(lane >> 3, 2), g = cGrid8[i];
+  const int no = ixe[i] - 1;
+  double h[3], hp[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int st = a == 0 ? 1 : a == 1 ? 3 : 9, up = (g >> a) & 1;
+    const int o = 2 * ((g & 1) + 3 * ((g >> 1) & 1) + 9 * (g >> 2));
+    const double* c = S.c[j];
+    const double own = c[o], mid = c[up ? o - st : o + st], opp = c[up ? o - 2 * st : o + 2 * st];
+    const double d = 2.0 * (own - mid) - 0.5 * (own - opp);
+    h[a] = up ? d : -d;
+    const int lo = g & ~(1 << a), hi = lo | (1 << a);
+    S.J[j][a][i] = 0.5 * (S.l[j][hi] - S.l[j][lo]);
+    hp[a] = 0.5 * (S.l[3][hi] - S.l[3][lo]);
+  }
+  __syncwarp();
+  const int j1 = j == 2 ? 0 : j + 1, j2 = j == 0 ? 2 : j - 1;
+  double ji[3], det = 0.0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const int p = (a + 1) % 3, q = (a + 2) % 3;
+    ji[a] = S.J[j1][p][i] * S.J[j2][q][i] - S.J[j2][p][i] * S.J[j1][q][i];
+    det += S.J[j][a][i] * ji[a];
+  }
+  if (__any_sync(0xffffffffu, !(det > 1.0e-14))) {
+    if (lane == 0) atomicOr(L.err, 1);
+    colour_wait();
+    return;
+  }
+  const double rd = 1.0 / det;
+  if constexpr (MODE == 7) {
+    // tx is the porosity change accumulator here
+    const double e = rd * (h[0] * ji[0] + h[1] * ji[1] + h[2] * ji[2]);
+    const double e1 = __shfl_sync(0xffffffffu, e, i + 8), e2 = __shfl_sync(0xffffffffu, e, i + 16);
+    colour_wait();
+    if (lane < 8) tx[no] += mc.coef_biot * (e + e1 + e2) + mc.imod_biot * S.l[3][g];
+  } else {
+    __syncwarp();
+    // (lanes 24..31 write what lanes 16..23 do)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) S.J[j][a][i] = ji[a];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      S.G[j][k][i] =
+          rd * (h[0] * S.J[k][0][i] + h[1] * S.J[k][1][i] + h[2] * S.J[k][2][i]);
+    const double gj = j == 0 ? L.g0 : j == 1 ? L.g1 : L.g2;
+    const double f =
+        mc.perm * (mc.fluid_d * gj - rd * (hp[0] * ji[0] + hp[1] * ji[1] + hp[2] * ji[2]));
+    __syncwarp();
+    const double sn = (S.G[j][j][i] + mc.b * S.G[j1][j1][i] + mc.b * S.G[j2][j2][i]) * mc.a -
+                      mc.coef_biot * dp[no];
+    const double sh = (S.G[j][j1][i] + S.G[j1][j][i]) * mc.c * mc.a;
+    colour_wait();
+    if (lane < 24) {  // components xx yy zz xy yz zx
+      double* T6 = tx + (size_t)6 * no;
+      double* B6 = txb + (size_t)6 * no;
+      T6[j] += sn;
+      B6[j] += sn + mc.coef_biot * S.l[3][g];
+      T6[3 + j] += sh;
+      B6[3 + j] += sh;
+      flux[(size_t)3 * no + j] += f;
     }
   }
 }

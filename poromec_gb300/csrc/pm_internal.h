@@ -89,6 +89,7 @@ struct ElemLaunch {
   const int32_t* elems;  // 1-based element ids of the colour
   int nelem;
   int nen;
+  bool chain;  // the stream's last launch is this pass's previous colour
   const int64_t* node_val_off;
   const int32_t* node_W;
   double dt, t;

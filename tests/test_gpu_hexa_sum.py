@@ -4,6 +4,7 @@ and its gradients, on distorted, flat and widely scaled elements."""
 import numpy as np
 import pytest
 
+import oracle
 import poromec_gb300 as pg
 from poromec_gb300 import meshgen
 
@@ -101,3 +102,64 @@ def test_against_the_assembled_matrix(n, jitter, scale):
     Kst = np.where(np.outer(isp, isp), K, 0.0) - Kperm
     gM = gr.cpu().numpy()[:, 2].sum()
     assert abs(gM - lam @ Kst @ xd) <= 1e-13 * np.abs(lam) @ (G @ np.abs(xd))
+
+
+def _distorted(n, jitter, scale):
+    pb = _problem(n, jitter, scale)
+    o = oracle.from_fixture(pb)
+    rng = np.random.default_rng(23)
+    u = 1e-3 * rng.standard_normal((int(pb["nnode"]), 4))
+    dp = 1e-3 * rng.standard_normal(int(pb["nnode"]))
+    return pb, o, pg.from_problem(pb), u, dp
+
+
+@pytest.mark.parametrize("n,jitter,scale", [(1, 0.2, (1, 1, 1)), (2, 0.15, (1, 1, 0.1)),
+                                            (3, 0.1, (1, 1, 1))])
+def test_vertices_against_the_oracle(n, jitter, scale):
+    """Nodal stresses and fluxes. A stress is some 20 terms,
+    each up to 1e2 of the largest result (a derivative against its differences):
+    20 x 100 x 2^-53 = 2e-13 of the largest."""
+    pb, o, m, u, dp = _distorted(n, jitter, scale)
+    m.set_state(u=u, u0=u, dp=dp)
+    o.set_state(u=u, u0=u, dp=dp)
+    kh = np.abs(np.asarray(pb["e"]).reshape(-1, oracle.PROP)[:, 2]).max()
+    for name, a, b in zip(("stress", "stressB", "stressE", "flux"), m.stress(), o.stress()):
+        s = max(np.abs(b).max(), kh if name == "flux" else 0.0)
+        assert np.abs(a - b).max() <= 2e-13 * s, name
+
+
+@pytest.mark.parametrize("n,jitter,kinds", [(1, 0.2, (40, 0)), (1, 0.2, (41, 43)),
+                                            (2, 0.15, (40, 43)), (3, 0.1, (41, 0))])
+def test_face_loads_against_the_oracle(n, jitter, kinds):
+    """Loads on all six faces of every element (a face is left out on every other element):
+    some 9 points x 6 faces x 8 elements of products a node, 64 x 20 of the state's
+    forces, 2^-53 each and some 10 operations deep: 1e-12 of the largest force."""
+    pb = _problem(n, jitter, (1, 1, 1))
+    numel, nf = int(pb["numel"]), np.asarray(pb["fload"]).shape[1]
+    load = np.array([[kinds[0], 0, 2], [kinds[1], 0, 2]], np.int32)
+    fload = np.zeros((2, nf, 2))
+    fload[:, 0] = [0.0, 5.0]
+    fload[:, 1] = [[1.0, 2.0], [3.0, 1.0]]
+    fload[:, 2] = [[-0.5, 0.3], [0.0, 0.0]]
+    fload[:, 3] = [[0.7, -2.0], [0.0, 0.0]]
+    eload = np.zeros((numel, 7), np.int32)
+    eload[:, :6] = 1
+    eload[::2, 3] = 0
+    eloadp = np.zeros((numel, 7), np.int32)
+    if kinds[1]:
+        eloadp[:, :6] = 2
+        eloadp[::2, 1] = 0
+    pb.update(load=load, fload=fload, eload=eload, eloadp=eloadp)
+    rng = np.random.default_rng(29)
+    u = 1e-3 * rng.standard_normal((int(pb["nnode"]), 4))
+    dp = 1e-3 * rng.standard_normal(int(pb["nnode"]))
+    m, o = pg.from_problem(pb), oracle.from_fixture(pb)
+    o.set_loads(eload=eload, eloadp=eloadp, load=load, fload=fload)
+    for t in (m, o):
+        t.set_env(pb["gravity"], float(pb["dt"]), 2.0)
+        t.set_state(u=u, u0=u, dp=dp)
+    b, bo = m.pform(4, False, True, u, np.zeros(m.neq)), np.zeros(o.neq)
+    o.pform(4, False, True, u, bo)
+    z = m.pform(4, False, True, u, np.zeros(m.neq))
+    assert np.array_equal(b, z)
+    assert np.abs(b - bo).max() <= 1e-12 * np.abs(bo).max()
