@@ -67,6 +67,25 @@ __device__ __forceinline__ T shfl(T v, int m) {
   return __shfl_xor_sync(0xffffffffu, v, m);
 }
 
+// Row sums of one node by lane t of its sub-warp, U columns a trip.  FP64
+// instructions bound the kernel only while enough loads are in flight for them, and
+// the compiler's own choice of U was not the best.  Microseconds per PCG iteration of
+// the 40^3 cube and the 20^3 tetra box (fused dot): its choice 385 and 78.6, 2 columns
+// 427 and 68.0, 3 344 and 68.0, 4 361 and 72.9, 5 362 and 66.7, 6 379 and 71.9.  The
+// plain product of the 56^3 cube: 830 its choice, 813 with 3, 800 with 5, and its
+// first one on new data 946, 997 and 907.
+template <typename T, int D, int U>
+__device__ __forceinline__ void spmv_rows(const T* __restrict__ v,
+                                          const int32_t* __restrict__ cols,
+                                          const T* __restrict__ x, int W, int t, T (&a)[4]) {
+#pragma unroll U
+  for (int c = t; c < W; c += kSub) {
+    const T xv = x[cols[c]];
+#pragma unroll
+    for (int r = 0; r < D; ++r) a[r] += v[r * W + c] * xv;
+  }
+}
+
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256)
     k_spmv(PanelView P, const T* __restrict__ val, const T* __restrict__ x,
@@ -78,51 +97,33 @@ __global__ void __launch_bounds__(256)
   const int t = lane & (kSub - 1);
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int nwarp = (int)((gridDim.x * blockDim.x) >> 5);
-  constexpr int kNodesPerWarp = 32 / kSub;
+  constexpr int kNodesPerWarp = 32 / kSub, U = MODE == 0 ? 5 : MODE == 4 ? 4 : 3;
   double dsum = 0.0;
   for (int base = warp * kNodesPerWarp; base < P.nact; base += nwarp * kNodesPerWarp) {
-    const NodeRef nr = node_ref(P, base + (lane >> 3));
-    int e0 = 0, d = 0, W = 0;
-    T a0 = T(0), a1 = T(0), a2 = T(0), a3 = T(0);
+    const NodeRef nr = node_ref(P, base + lane / kSub);
+    int e0 = 0, d = 0;
+    T a[4] = {T(0), T(0), T(0), T(0)};
     if (nr.on) {
       e0 = nr.e0;
       d = nr.d;
-      W = nr.W;
       const T* v = val + nr.vo;
       const int32_t* cols = P.cols + nr.co;
-      if (d == 4) {
-        for (int c = t; c < W; c += kSub) {
-          const T xv = x[cols[c]];
-          a0 += v[c] * xv;
-          a1 += v[W + c] * xv;
-          a2 += v[2 * W + c] * xv;
-          a3 += v[3 * W + c] * xv;
-        }
-      } else if (d == 3) {
-        for (int c = t; c < W; c += kSub) {
-          const T xv = x[cols[c]];
-          a0 += v[c] * xv;
-          a1 += v[W + c] * xv;
-          a2 += v[2 * W + c] * xv;
-        }
-      } else {
-        for (int c = t; c < W; c += kSub) {
-          const T xv = x[cols[c]];
-          a0 += v[c] * xv;
-          if (d > 1) a1 += v[W + c] * xv;
-        }
-      }
+      if (d == 4) spmv_rows<T, 4, U>(v, cols, x, nr.W, t, a);
+      else if (d == 3) spmv_rows<T, 3, U>(v, cols, x, nr.W, t, a);
+      else if (d == 2) spmv_rows<T, 2, U>(v, cols, x, nr.W, t, a);
+      else spmv_rows<T, 1, U>(v, cols, x, nr.W, t, a);
     }
     // transposed butterfly over the 8 lanes of the sub-warp
-    const bool h4 = (t & 4) != 0, h2 = (t & 2) != 0;
-    T k0 = h4 ? a2 : a0, k1 = h4 ? a3 : a1;
-    k0 += shfl(h4 ? a0 : a2, 4);
-    k1 += shfl(h4 ? a1 : a3, 4);
+    constexpr int o1 = kSub / 2, o2 = kSub / 4;
+    const bool h1 = (t & o1) != 0, h2 = (t & o2) != 0;
+    T k0 = h1 ? a[2] : a[0], k1 = h1 ? a[3] : a[1];
+    k0 += shfl(h1 ? a[0] : a[2], o1);
+    k1 += shfl(h1 ? a[1] : a[3], o1);
     T k = h2 ? k1 : k0;
-    k += shfl(h2 ? k0 : k1, 2);
+    k += shfl(h2 ? k0 : k1, o2);
     k += shfl(k, 1);
-    const int r = (h4 ? 2 : 0) + (h2 ? 1 : 0);
-    if ((t & 1) == 0 && r < d) {
+    const int r = (h1 ? 2 : 0) + (h2 ? 1 : 0);
+    if ((t & (o2 - 1)) == 0 && r < d) {
       y[e0 + r] = k;
       if (MODE == 4) dsum += double(k) * xd[e0 + r];
       else if (MODE != 0) dsum += double(k * x[e0 + r]);
