@@ -547,12 +547,12 @@ cudaError_t launch(const PanelView& P, const double* val, CoopArgs A, int grid, 
 // extra FP64 instruction per column costs more than the exchange.  Microseconds
 // per PCG iteration (fused warp per node / two nodes per warp / phase kernels):
 // column 2 x 2 x 40 10.0 / 14.3 / 25.7, cube 8^3 14.2 / 15.1 / 24.0, cube 12^3
-// 23.6 / 21.1 / 29.3, tetra 11^3 21.3 / 20.1 / 28.5.
+// 23.6 / 21.1 / 28.2, tetra 11^3 21.3 / 20.1 / 28.4.
 constexpr int kFuseNodes = 32;
 // Above this many panel values per CTA the FP64 pipe hides the phase kernels'
 // launches and feeds better from their many CTAs: cube 16^3 (70 k values per
-// CTA) 43.1 against 44.7 us, tetra 16^3 (61 k) 38.0 against 45.4, cube 20^3
-// (135 k) 83 against 68, tetra 20^3 (124 k) 81 against 79.
+// CTA) 38.4 against 43.7 us, tetra 16^3 (63 k) 38.3 against 41.3, tetra 20^3
+// (124 k) 81 against 68.
 constexpr int64_t kCoopValues = 80000;
 
 // at least a node per scheduler

@@ -86,7 +86,7 @@ __device__ __forceinline__ void spmv_rows(const T* __restrict__ v,
   }
 }
 
-template <typename T, int MODE>
+template <typename T, int MODE, int U>
 __global__ void __launch_bounds__(256)
     k_spmv(PanelView P, const T* __restrict__ val, const T* __restrict__ x,
            T* __restrict__ y, KrylovScalars* ks, double* partial, unsigned* counter,
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(256)
   const int t = lane & (kSub - 1);
   const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int nwarp = (int)((gridDim.x * blockDim.x) >> 5);
-  constexpr int kNodesPerWarp = 32 / kSub, U = MODE == 0 ? 5 : MODE == 4 ? 4 : 3;
+  constexpr int kNodesPerWarp = 32 / kSub;
   double dsum = 0.0;
   for (int base = warp * kNodesPerWarp; base < P.nact; base += nwarp * kNodesPerWarp) {
     const NodeRef nr = node_ref(P, base + lane / kSub);
@@ -1484,11 +1484,18 @@ cudaError_t spmv(const PanelView& P, const double* val64, const double* x, doubl
   // small mesh launches only the CTAs it fills, and its fused dot sums that
   // many partials
   const int grid = std::max(1, std::min(kRedBlocks, (P.nact + 31) / 32));
+  // columns per trip (spmv_rows); with few nodes 4, as the compiler had it: the
+  // product of the 3^3 cube takes 7.4 us then and 7.7 with 5 (10^3: 14.4 and 15.3,
+  // 16^3, 18,785 nodes, 30.4 and 31.3; tetra 14^3, 24,389 nodes, 22.6 and 20.5)
+  const bool many = P.nact >= 24000;
+  auto run = [&](auto few, auto most) {
+    (many ? most : few)<<<grid, 256, 0, s>>>(P, val64, x, y, ks, partial, counter, nullptr);
+  };
   switch (mode) {
-    case 0: k_spmv<double, 0><<<grid, 256, 0, s>>>(P, val64, x, y, ks, partial, counter); break;
-    case 1: k_spmv<double, 1><<<grid, 256, 0, s>>>(P, val64, x, y, ks, partial, counter); break;
-    case 2: k_spmv<double, 2><<<grid, 256, 0, s>>>(P, val64, x, y, ks, partial, counter); break;
-    default: k_spmv<double, 3><<<grid, 256, 0, s>>>(P, val64, x, y, ks, partial, counter); break;
+    case 0: run(k_spmv<double, 0, 4>, k_spmv<double, 0, 5>); break;
+    case 1: run(k_spmv<double, 1, 4>, k_spmv<double, 1, 3>); break;
+    case 2: run(k_spmv<double, 2, 4>, k_spmv<double, 2, 3>); break;
+    default: run(k_spmv<double, 3, 4>, k_spmv<double, 3, 3>); break;
   }
   return cudaGetLastError();
 }
@@ -1504,7 +1511,7 @@ cudaError_t pcgm_init(int n, const double* b, const double* m, KrylovVecs& V,
 cudaError_t pcgm_iteration(const PanelView& P, const float* val32, int n, const double* m,
                            KrylovVecs& V, KrylovVecs32& V32, KrylovScalars* ks,
                            double* partial, unsigned* counter, cudaStream_t s) {
-  k_spmv<float, 4><<<kRedBlocks, 256, 0, s>>>(P, val32, V32.p, V32.q, ks, partial, counter,
+  k_spmv<float, 4, 4><<<kRedBlocks, 256, 0, s>>>(P, val32, V32.p, V32.q, ks, partial, counter,
                                                V.p);
   k_pcgm_update<<<vec_grid(n), 256, 0, s>>>(n, V.x, V.p, V.r, V32.q, m, V.z, ks, partial,
                                              counter);
