@@ -78,7 +78,7 @@ template <typename T, int D, int U>
 __device__ __forceinline__ void spmv_rows(const T* __restrict__ v,
                                           const int32_t* __restrict__ cols,
                                           const T* __restrict__ x, int W, int t, T (&a)[4]) {
-#pragma unroll U
+#pragma unroll(U > 0 ? U : 1)
   for (int c = t; c < W; c += kSub) {
     const T xv = x[cols[c]];
 #pragma unroll
@@ -101,9 +101,38 @@ __global__ void __launch_bounds__(256)
   double dsum = 0.0;
   for (int base = warp * kNodesPerWarp; base < P.nact; base += nwarp * kNodesPerWarp) {
     const NodeRef nr = node_ref(P, base + lane / kSub);
-    int e0 = 0, d = 0;
-    T a[4] = {T(0), T(0), T(0), T(0)};
-    if (nr.on) {
+    int e0 = 0, d = 0, W = 0;
+    T a0 = T(0), a1 = T(0), a2 = T(0), a3 = T(0);
+    if (U == 0 && nr.on) {  // few nodes: loops as the compiler has them
+      e0 = nr.e0;
+      d = nr.d;
+      W = nr.W;
+      const T* v = val + nr.vo;
+      const int32_t* cols = P.cols + nr.co;
+      if (d == 4) {
+        for (int c = t; c < W; c += kSub) {
+          const T xv = x[cols[c]];
+          a0 += v[c] * xv;
+          a1 += v[W + c] * xv;
+          a2 += v[2 * W + c] * xv;
+          a3 += v[3 * W + c] * xv;
+        }
+      } else if (d == 3) {
+        for (int c = t; c < W; c += kSub) {
+          const T xv = x[cols[c]];
+          a0 += v[c] * xv;
+          a1 += v[W + c] * xv;
+          a2 += v[2 * W + c] * xv;
+        }
+      } else {
+        for (int c = t; c < W; c += kSub) {
+          const T xv = x[cols[c]];
+          a0 += v[c] * xv;
+          if (d > 1) a1 += v[W + c] * xv;
+        }
+      }
+    } else if (nr.on) {
+      T a[4] = {T(0), T(0), T(0), T(0)};
       e0 = nr.e0;
       d = nr.d;
       const T* v = val + nr.vo;
@@ -112,13 +141,17 @@ __global__ void __launch_bounds__(256)
       else if (d == 3) spmv_rows<T, 3, U>(v, cols, x, nr.W, t, a);
       else if (d == 2) spmv_rows<T, 2, U>(v, cols, x, nr.W, t, a);
       else spmv_rows<T, 1, U>(v, cols, x, nr.W, t, a);
+      a0 = a[0];
+      a1 = a[1];
+      a2 = a[2];
+      a3 = a[3];
     }
     // transposed butterfly over the 8 lanes of the sub-warp
     constexpr int o1 = kSub / 2, o2 = kSub / 4;
     const bool h1 = (t & o1) != 0, h2 = (t & o2) != 0;
-    T k0 = h1 ? a[2] : a[0], k1 = h1 ? a[3] : a[1];
-    k0 += shfl(h1 ? a[0] : a[2], o1);
-    k1 += shfl(h1 ? a[1] : a[3], o1);
+    T k0 = h1 ? a2 : a0, k1 = h1 ? a3 : a1;
+    k0 += shfl(h1 ? a0 : a2, o1);
+    k1 += shfl(h1 ? a1 : a3, o1);
     T k = h2 ? k1 : k0;
     k += shfl(h2 ? k0 : k1, o2);
     k += shfl(k, 1);
@@ -1484,18 +1517,18 @@ cudaError_t spmv(const PanelView& P, const double* val64, const double* x, doubl
   // small mesh launches only the CTAs it fills, and its fused dot sums that
   // many partials
   const int grid = std::max(1, std::min(kRedBlocks, (P.nact + 31) / 32));
-  // columns per trip (spmv_rows); with few nodes 4, as the compiler had it: the
-  // product of the 3^3 cube takes 7.4 us then and 7.7 with 5 (10^3: 14.4 and 15.3,
-  // 16^3, 18,785 nodes, 30.4 and 31.3; tetra 14^3, 24,389 nodes, 22.6 and 20.5)
+  // columns per trip (spmv_rows); with few nodes the compiler's loops: the product
+  // of the 3^3 cube takes 7.4 us with them, 7.7 to 8.1 with 4 or 5 (10^3: 14.4 and
+  // 15.3; 16^3, 18,785 nodes, 30.8 and 31.3; tetra 14^3, 24,389 nodes, 23.2 and 20.5)
   const bool many = P.nact >= 24000;
   auto run = [&](auto few, auto most) {
     (many ? most : few)<<<grid, 256, 0, s>>>(P, val64, x, y, ks, partial, counter, nullptr);
   };
   switch (mode) {
-    case 0: run(k_spmv<double, 0, 4>, k_spmv<double, 0, 5>); break;
-    case 1: run(k_spmv<double, 1, 4>, k_spmv<double, 1, 3>); break;
-    case 2: run(k_spmv<double, 2, 4>, k_spmv<double, 2, 3>); break;
-    default: run(k_spmv<double, 3, 4>, k_spmv<double, 3, 3>); break;
+    case 0: run(k_spmv<double, 0, 0>, k_spmv<double, 0, 5>); break;
+    case 1: run(k_spmv<double, 1, 0>, k_spmv<double, 1, 3>); break;
+    case 2: run(k_spmv<double, 2, 0>, k_spmv<double, 2, 3>); break;
+    default: run(k_spmv<double, 3, 0>, k_spmv<double, 3, 3>); break;
   }
   return cudaGetLastError();
 }
@@ -1511,7 +1544,7 @@ cudaError_t pcgm_init(int n, const double* b, const double* m, KrylovVecs& V,
 cudaError_t pcgm_iteration(const PanelView& P, const float* val32, int n, const double* m,
                            KrylovVecs& V, KrylovVecs32& V32, KrylovScalars* ks,
                            double* partial, unsigned* counter, cudaStream_t s) {
-  k_spmv<float, 4, 4><<<kRedBlocks, 256, 0, s>>>(P, val32, V32.p, V32.q, ks, partial, counter,
+  k_spmv<float, 4, 0><<<kRedBlocks, 256, 0, s>>>(P, val32, V32.p, V32.q, ks, partial, counter,
                                                V.p);
   k_pcgm_update<<<vec_grid(n), 256, 0, s>>>(n, V.x, V.p, V.r, V32.q, m, V.z, ks, partial,
                                              counter);
