@@ -22,8 +22,8 @@
 // FP64 instructions set the rest: a dependent add takes 66 clocks and occupies
 // the scheduler's pipe for 64 whatever its mask, a division 1,430.  So the
 // reductions and the scalar recurrences run in one warp, the quotients come from
-// a Newton iteration (alpha) or a reciprocal formed ahead (beta), and the results
-// are broadcast.  The panels are read through L1, which holds them from one
+// a reciprocal by Newton's iteration, formed ahead where the divisor is known, and
+// a correction, and the results are broadcast.  The panels are read through L1, which holds them from one
 // iteration to the next where they fit.
 //
 // The recurrences and tests are those of the kernels in pm_sparse.cu
@@ -214,11 +214,14 @@ __device__ __forceinline__ double recip(double a) {
   x = fma(x, fma(-a, x, 1.0), x);
   return fma(x, fma(-a, x, 1.0), x);
 }
-// b / a with one correction of the quotient's remainder
-__device__ __forceinline__ double quotient(double b, double a) {
-  const int e = (__double2hiint(b) >> 20) & 0x7ff;
-  const double x = recip(a);
-  if (e < 200 || e > 1846 || !isfinite(x)) return b / a;
+// b / a from x = recip(a), formed ahead or not, with one correction by the
+// remainder (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34, 1990): the quotient's own rounding
+// is what is left of its error, as in the division.  The division itself where x,
+// the quotient or the remainder could leave the normal range.
+__device__ __forceinline__ double quotient(double b, double a, double x) {
+  const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
+  if (ea < 100 || ea > 1946 || eb < 200 || eb > 1846 || abs(eb - ea) > 900) return b / a;
   const double q = b * x;
   return fma(fma(-a, q, b), x, q);
 }
@@ -318,7 +321,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
   const int maxit = ks->maxit;
   // |d| at or above this is not converged whatever the rounding of the root
   const double far = conv * conv * (1.0 + 1e-9);
-  double d = ks->d, rd = 1.0 / d;
+  double d = ks->d, rd = recip(d);
   unsigned long long epoch = A.epoch;
   int iter = 0;
   double pq = 0.0, beta = 0.0, alpha = 0.0;
@@ -333,7 +336,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
     bool ok = exchange<1>(S, A, X.rows, ++epoch, tot);
     if (threadIdx.x < 32) {
       pq = tot[0];
-      alpha = quotient(d, pq);
+      alpha = quotient(d, pq, recip(pq));
       if (threadIdx.x == 0) {
         S.scal[0] = alpha;
         S.flag = isfinite(alpha) ? 0 : 3;  // (p, A p) = 0: x stays as it is
@@ -355,7 +358,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
     ok = exchange<1, FUSE>(S, A, X.rows, ++epoch, tot);
     if (threadIdx.x < 32) {
       const double di = tot[0];
-      beta = di * rd;
+      beta = quotient(di, d, rd);
       d = di;
       ++iter;
       if (threadIdx.x == 0) {
@@ -416,7 +419,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
   const double conv = ks->conv;
   const int maxit = ks->maxit;
   double rho = ks->d, tau = ks->normr, vj = ks->neta, nr = 0.0, sigma = 0.0, alpha = 0.0;
-  double rrho = 1.0 / rho, rtau = 1.0 / tau;
+  double rrho = recip(rho), rtau = recip(tau);
   unsigned long long epoch = A.epoch;
   int iter = 0;
   double *pn = A.p, *po = A.p2;
@@ -433,7 +436,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
     bool ok = exchange<1>(S, A, X.rows, ++epoch, tot1);
     if (threadIdx.x < 32) {
       sigma = tot1[0];
-      alpha = quotient(rho, sigma);
+      alpha = quotient(rho, sigma, recip(sigma));
       if (threadIdx.x == 0) {
         S.scal[0] = alpha;
         if (!ok) S.stop = ks->fault = 1;
@@ -459,10 +462,11 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
     ok = exchange<2, FUSE>(S, A2, X.rows, ++epoch, tot);
     if (threadIdx.x < 32) {
       nr = sqrt(tot[0]);
-      const double vn = nr * rtau;
+      const double vn = quotient(nr, tau, rtau);
       const double cn2 = recip(1.0 + vn * vn);
       tau = tau * vn * sqrt(cn2);
-      const double t1 = cn2 * vj * vj, t2 = cn2 * alpha, beta = tot[1] * rrho;
+      const double t1 = cn2 * vj * vj, t2 = cn2 * alpha,
+                   beta = quotient(tot[1], rho, rrho);
       vj = vn;
       ++iter;
       if (threadIdx.x == 0) {

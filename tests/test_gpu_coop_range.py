@@ -1,0 +1,35 @@
+"""The cooperative FP64 solve (pm_coop.cu) on right-hand sides whose inner
+products are at the lower end of the doubles."""
+import numpy as np
+import pytest
+
+import poromec_gb300 as pg
+from poromec_gb300 import meshgen
+
+pytestmark = pytest.mark.gpu
+
+
+def _assembled(n):
+    m = pg.from_problem(meshgen.cube_problem(n=n))
+    m.pform(2, True, False, np.zeros((m.nnode, 4)), None)
+    return m
+
+
+# the fused form and the one with two nodes per warp
+@pytest.mark.parametrize("solver", [1, 11])
+@pytest.mark.parametrize("n", [3, 11])
+def test_inner_products_below_the_normal_range(n, solver):
+    """b scaled by a power of two until its larger inner product is 1e-300, solved
+    to 1e-5: the products end near 1e-310, where the reciprocal of a product is no
+    longer a double but the quotient of two is. The stopping test holds for the
+    scaled-back solution with the margin of the other solver tests."""
+    m = _assembled(n)
+    ia, ja, ad, al = m.get_csrd()
+    b = np.random.default_rng(n).standard_normal(m.neq)
+    s = 2.0 ** np.round(0.5 * np.log2(1e-300 / max(b @ b, abs(np.sum(b * b / ad)))))
+    tol = 1e-5
+    x, info = m.solve(b * s, solver=solver, precond=2, tol=tol, maxit=20000)
+    r = b - m.matvec(x / s)
+    w = np.ones_like(ad) if solver == 11 else 1.0 / ad
+    assert info.iters > 1
+    assert np.sqrt(abs(np.sum(r * r * w))) <= 1.1 * tol * np.sqrt(abs(np.sum(b * b * w)))
