@@ -319,8 +319,9 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
   KrylovScalars* ks = A.ks;
   const double conv = ks->conv;
   const int maxit = ks->maxit;
-  // |d| at or above this is not converged whatever the rounding of the root
-  const double far = conv * conv * (1.0 + 1e-9);
+  // |d| at or above this is not converged whatever the rounding of the root (where
+  // the square has all its bits: below, the root decides)
+  const double far = conv * conv >= 1e-280 ? conv * conv * (1.0 + 1e-9) : INFINITY;
   double d = ks->d, rd = recip(d);
   unsigned long long epoch = A.epoch;
   int iter = 0;

@@ -33,3 +33,30 @@ def test_inner_products_below_the_normal_range(n, solver):
     w = np.ones_like(ad) if solver == 11 else 1.0 / ad
     assert info.iters > 1
     assert np.sqrt(abs(np.sum(r * r * w))) <= 1.1 * tol * np.sqrt(abs(np.sum(b * b * w)))
+
+
+def test_tolerance_whose_square_is_no_double():
+    """b = A v for an eigenvector v of D^-1 A (D the diagonal of A): PCG's first step
+    is exact. Scaled so that (r, z) starts near 1e-318, five digits of a double, it
+    ends at 0 and the target, 1e-4 of its root, squares to 0: converged after one
+    iteration. A product is some 2e5 units of the smallest double and each of its terms
+    is rounded by half of one, so x is within 2 neq / 2 / 2e5 < 2e-3 of v."""
+    import scipy.linalg
+    m = _assembled(2)
+    ia, ja, ad, al = m.get_csrd()
+    A = np.diag(ad)
+    rows = np.repeat(np.arange(m.neq), np.diff(ia))
+    A[rows, ja - 1] = al
+    A[ja - 1, rows] = al
+    lam, V = scipy.linalg.eig(A / ad[:, None])
+    real = np.abs(lam.imag) <= 1e-12 * np.abs(lam)
+    V, lam = V.real[:, real], lam.real[real]
+    # the eigenvector with the largest (b, D^-1 b) for its entries: no cancellation
+    b = A @ V
+    k = np.argmax(np.abs(np.sum(b * b / ad[:, None], 0)) / np.sum(b * b / np.abs(ad[:, None]), 0))
+    v, b = V[:, k], b[:, k]
+    s = 2.0 ** np.round(0.5 * np.log2(1e-318 / abs(np.sum(b * b / ad))))
+    x, info = m.solve(b * s, solver=1, precond=2, tol=1e-4, maxit=50)
+    assert info.iters == 1
+    assert m.neq <= 400
+    assert np.abs(x / s - v).max() <= 2e-3 * np.abs(v).max()
