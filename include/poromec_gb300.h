@@ -281,7 +281,9 @@ int pm_adjoint_grad_dev(pm_handle h, const double* d_lam, const double* d_un,
  * [4] Krylov iterations of all the solves of the last single-mesh
  * pm_step (the step's info->iters counts its last solve only; 0 for a batch),
  * [5] device time of the last Krylov solve,
- * [6] Krylov iterations of the last solve, [7] kernels launched by the step. */
+ * [6] Krylov iterations of the last solve, [7] kernels launched by the step,
+ * [8] form of the last Krylov solve: 1 or 2 one cooperative kernel (a warp per
+ * node, two nodes per warp), 0 a kernel per phase. */
 int pm_get_timers(pm_handle h, double* t, int n);
 
 /* ---- input decks ---------------------------------------------------------

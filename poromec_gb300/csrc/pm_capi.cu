@@ -523,8 +523,10 @@ int run_coop(Handle* h, bool sqmr, pm::KrylovScalars* ks, Coop* how) {
     }
     PM_CUDA(cudaMemsetAsync(h->D.coop, 0, pm::coop_scratch_bytes(), h->stream));
   }
+  int polls = pm::kCoopPolls;  // PM_COOP_POLLS overrides
+  if (const char* e = std::getenv("PM_COOP_POLLS")) polls = std::atoi(e);
   if (pm::krylov_coop(sqmr, h->P.view(), h->P.val, h->D.m, h->D.kv, h->D.ks, h->D.coop,
-                      h->coop_epoch, h->sms, h->stream) != cudaSuccess) {
+                      h->coop_epoch, polls, h->sms, h->stream) != cudaSuccess) {
     cudaGetLastError();  // the refusal is not this solve's error
     h->coop_failed = true;
     return PM_OK;
@@ -534,6 +536,7 @@ int run_coop(Handle* h, bool sqmr, pm::KrylovScalars* ks, Coop* how) {
   const bool done = ks->fault == 0 && ks->conv_flag != 0;
   h->coop_epoch += (unsigned long long)pm::kCoopEpochs * (ks->iter + 1);
   *how = done ? Coop::kSolved : Coop::kGaveUp;
+  if (done) h->timers[8] = pm::coop_form(h->P.view(), h->sms);
   if (!done) {
     h->coop_failed = true;
     if (h->debug) fprintf(stderr, "cooperative solve gave up: phase kernels\n");
@@ -565,6 +568,7 @@ int krylov(Handle* h, int solver, const double* d_b, double* d_x, double tol, in
   pm::KrylovScalars ks{};
   int sweeps = 0;
   double final_target = -1.0;  // compensated MINRES: the target its cycles refine to
+  h->timers[8] = 0.0;
   cudaEvent_t e0 = h->ev[0], e1 = h->ev[1];
   PM_CUDA(cudaEventRecord(e0, h->stream));
   if (solver == 1) {
@@ -2576,7 +2580,7 @@ int pm_adjoint_grad_dev(pm_handle hh, const double* d_lam, const double* d_un,
 int pm_get_timers(pm_handle hh, double* t, int n) {
   Handle* h = reinterpret_cast<Handle*>(hh);
   if (!h || !t) return PM_E_ARG;
-  for (int i = 0; i < n && i < 8; ++i) t[i] = h->timers[i];
+  for (int i = 0; i < n && i < 9; ++i) t[i] = h->timers[i];
   return PM_OK;
 }
 

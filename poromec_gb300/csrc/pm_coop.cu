@@ -44,7 +44,6 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kCoopMaxCtas = 160;            // senders and receivers of an exchange
 constexpr int kReplicas = 32;                // arrays of slots (at most one per lane)
-constexpr int kPollLimit = 1 << 22;          // about 2 s of polling
 
 // A form of the solve: LANES per node; FUSE, the exchange saved; THREADS per CTA, of
 // which CTAS are resident per SM; CHUNK columns per lane whose loads are in flight.
@@ -83,6 +82,7 @@ struct CoopArgs {
   KrylovScalars* ks;
   Slot* slots;
   unsigned long long epoch;  // the slots' last epoch
+  int polls;                 // of one exchange, before a CTA gives up
 };
 
 // The CTA's shared memory: partial sums, the recurrence's scalars (thread 0 keeps
@@ -266,7 +266,7 @@ __device__ __forceinline__ bool exchange(CoopShared<T>& S, const CoopArgs& A, in
   // all of a lane's slots in flight together: an exchange then costs one or two
   // load latencies, not one per slot
   bool late = true;
-  for (int n = 0; n < kPollLimit && late; ++n) {
+  for (int n = 0; n < A.polls && late; ++n) {
     unsigned long long e[kPer];
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
@@ -589,6 +589,10 @@ size_t coop_scratch_bytes() {
   return 6 * (size_t)kReplicas * kCoopMaxCtas * sizeof(Slot);
 }
 
+int coop_form(const PanelView& P, int sms) {
+  return P.nact <= kFuseNodes * coop_grid(P, sms) ? 1 : 2;
+}
+
 bool coop_fits(const PanelView& P, int64_t nnz, int sms) {
   if (sms < 1 || P.nact < 1) return false;
   const int grid = coop_grid(P, sms);
@@ -598,7 +602,7 @@ bool coop_fits(const PanelView& P, int64_t nnz, int sms) {
 
 cudaError_t krylov_coop(bool sqmr, const PanelView& P, const double* val, const double* m,
                         KrylovVecs& V, KrylovScalars* ks, void* scratch,
-                        unsigned long long epoch, int sms, cudaStream_t s) {
+                        unsigned long long epoch, int polls, int sms, cudaStream_t s) {
   const cudaError_t e = cudaMemsetAsync(&ks->fault, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
   CoopArgs A{};
@@ -611,8 +615,9 @@ cudaError_t krylov_coop(bool sqmr, const PanelView& P, const double* val, const 
   A.ks = ks;
   A.slots = static_cast<Slot*>(scratch);
   A.epoch = epoch;
+  A.polls = polls;
   const int grid = coop_grid(P, sms);
-  if (P.nact <= kFuseNodes * grid)
+  if (coop_form(P, sms) == 1)
     return sqmr ? launch<true, Fused>(P, val, A, grid, s) : launch<false, Fused>(P, val, A, grid, s);
   return sqmr ? launch<true, Pairs>(P, val, A, grid, s) : launch<false, Pairs>(P, val, A, grid, s);
 }

@@ -233,7 +233,7 @@ struct Handle {
   pm::BatchStepArrays bsa{};
   cudaGraphExec_t bstep_exec = nullptr;
   bool bstep_failed = false;
-  double timers[8] = {0};
+  double timers[9] = {0};
   int64_t launches = 0;        // kernels launched by the library (all calls)
   std::string err;
 };

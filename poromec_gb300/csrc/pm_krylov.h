@@ -155,15 +155,19 @@ cudaError_t sqmr_iteration(const PanelView& P, const double* val64, int n, const
 // kernel (pm_coop.cu) on at most sms CTAs.  scratch holds coop_scratch_bytes(),
 // zero before its first use; epoch is larger than any the earlier solves on it
 // reached (kCoopEpochs per iteration).
-// The flags are in *ks; ks->fault set or conv_flag 0: not solved.
+// The flags are in *ks; ks->fault set or conv_flag 0: not solved (a CTA saw another's
+// sum not arrive within so many polls).
 // coop_fits: whether this form is the faster one for a mesh of nnz panel values.
+// coop_form: 1 a warp per node, 2 two nodes per warp.
 constexpr int kCoopMaxSmem = 200 * 1024;
 constexpr int kCoopEpochs = 3;
+constexpr int kCoopPolls = 1 << 22;  // about 2 s
 size_t coop_scratch_bytes();
 bool coop_fits(const PanelView& P, int64_t nnz, int sms);
+int coop_form(const PanelView& P, int sms);
 cudaError_t krylov_coop(bool sqmr, const PanelView& P, const double* val, const double* m,
                         KrylovVecs& V, KrylovScalars* ks, void* scratch,
-                        unsigned long long epoch, int sms, cudaStream_t s);
+                        unsigned long long epoch, int polls, int sms, cudaStream_t s);
 // GMRES(l) vector kernels (pm_gmres.cu)
 cudaError_t gm_resid(int n, const double* b, const double* ax, const double* m, double* g1,
                      double* out, double* partial, unsigned* counter, cudaStream_t s);

@@ -32,8 +32,8 @@ def _product(m):
     return ad, lambda x: ad * x + L @ x + L.T @ x
 
 
-# nodes: 20, 81, 3,781 (25 per SM), 4,961 (33 per SM), 18,785; panel values
-# 10.6 M (16^3) and 12.7 M (17^3) on either side of 152 x 80,000
+# nodes: 20, 81, 3,700 (23 active ones per SM), 4,961 (31), 18,785 (120); panel values
+# 10.6 M (16^3) and 12.7 M (17^3), above the 152 x 65,000 of the cooperative solve
 @pytest.mark.parametrize("solver", [1, 11])
 @pytest.mark.parametrize("kind,n", [("column", 1), ("cube", 2), ("cube", 9), ("cube", 10),
                                     ("tetra", 4), ("cube", 16), ("cube", 17)])
