@@ -265,8 +265,9 @@ __device__ __forceinline__ bool exchange(CoopShared<T>& S, const CoopArgs& A, in
   double got[kPer];
   // all of a lane's slots in flight together: an exchange then costs one or two
   // load latencies, not one per slot
-  bool late = true;
-  for (int n = 0; n < A.polls && late; ++n) {
+  bool late;
+  int left = A.polls;
+  do {
     unsigned long long e[kPer];
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
@@ -277,8 +278,8 @@ __device__ __forceinline__ bool exchange(CoopShared<T>& S, const CoopArgs& A, in
     late = false;
 #pragma unroll
     for (int j = 0; j < kPer; ++j) late |= e[j] != epoch;
-  }
-  if (__any_sync(kFull, late)) return false;
+  } while (late && --left > 0);
+  if (__any_sync(kFull, late || A.polls <= 0)) return false;
   if (VIS) __threadfence();
   if (NV > 0) {
     double sum = 0.0;
