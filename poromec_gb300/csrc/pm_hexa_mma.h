@@ -1,5 +1,5 @@
-// pm_hexa_mma.h -- hexa20 element matrices on the FP16 tensor pipe, exact to
-// FP64 (included by pm_elements.cu inside its unnamed namespace).
+// pm_hexa_mma.h -- hexa20 element matrices on the FP16 tensor pipe, as accurate as
+// FP64 sums (included by pm_elements.cu inside its unnamed namespace).
 //
 // What bounds it.  All the matrix needs from the 64 points are the products
 //   P(r, c) = sum_g X_r(g) X_c(g)
@@ -9,16 +9,22 @@
 // instructions are no faster here.  mma.sync with FP16 operands and FP32 sums
 // does 1,017 multiply-adds per clock and SM (measured; int8 252).
 //
-// Split.  Each X is a 54-bit integer q (every value within a factor 2 of the
-// largest of its kind is held exactly, smaller ones to 2^-54 of it), cut into
+// Split.  Each X is a 54-bit integer q (every value within a factor 2 of its row's
+// largest is held exactly, smaller ones to 2^-54 of it), cut into
 // 7 balanced base-256 digits (Ozaki, Ogita, Oishi and Rump, "Error-free
 // transformations of matrix multiplication", Numer. Algorithms 59, 2012).
 // Digits are exact in FP16, their products are at most 2^14, and the sums
 // of all pairs s + t = d over 64 points stay below 2^23: exact in FP32.  The
 // 34 pairs with s + t <= 7 are kept; the dropped ones are 2^-59 of the largest
-// product, the final 64-bit integer's last place 2^-52.  (Without s + t = 7 the
-// entries' error against 64 bits was 1.6 times that of the DFMA sums.)  The kinds
-// (three directions, Np) have an exponent each, the largest of the element.
+// product, the final 64-bit integer's last place 2^-54 to 2^-56.  (Without s + t = 7
+// the entries' error against 64 bits was 1.6 times that of the DFMA sums.)
+//
+// Error.  Every row has its own exponent, so the error of P(r, c) is relative to
+// sqrt(P(r, r) P(c, c)) whatever the element's shape: at most 1.4e-16 of it, where
+// FP64 sums have up to 1.3e-15, on cubes, jittered elements and thicknesses that
+// taper from 1 to 1e-1 .. 1e-6 between opposite corners.  (With one exponent for all
+// derivatives of a direction, and a last place of 2^-50 to 2^-52, it was 1.4e-14 at
+// 1e-2 and 7e-12 at 1e-4.)
 //
 // Per element: 256 threads (geometry: 4 threads per point, then 28 tiles of
 // 16 x 8 over 8 warps, then a node pair per thread), two elements per SM.
@@ -33,6 +39,7 @@ constexpr int kHxStride = 72;   // halves per digit row of 64 points: no bank co
 constexpr int kHxDig = 7;
 constexpr int kHxSum = 8;       // digit pairs kept: s + t < kHxSum
 constexpr int kHxPs = 69;       // doubles per row of P
+constexpr int kHxBad = 1 << 14; // exponent of a row with a value that is not finite
 constexpr int kHxSlots = 28;    // product slots per row: 20 nodes, 8 vertices
 
 struct SmHx {
@@ -53,8 +60,8 @@ struct SmHx {
   int nodes[20], mat;
   int eq[20][kNdf], e0[20], W[20];
   int64_t off[20];
-  int em[4];                       // largest exponent: d/dx, d/dy, d/dz, Np
-  int fail, bad;
+  int em[kHxRows];                 // largest exponent of each row
+  int fail;
 };
 
 __device__ __forceinline__ int hx_exp(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
@@ -102,7 +109,7 @@ __device__ __forceinline__ void hx_ldsm(unsigned (&r)[4], const unsigned short* 
 
 // Rows ra .. ra + 15 times rows rb .. rb + 7 over the 64 points: the lane's
 // four entries (row g, g, g + 8, g + 8 with g = lane / 4; column 2 (lane % 4),
-// + 1, ...) as integers in units of 2^56 of q q.
+// + 1, ...) as integers below 2^62 in units of 2^52 of q q.
 __device__ __forceinline__ void hx_tile(const SmHx& S, int ra, int rb, int lane,
                                         long long (&out)[4]) {
   float acc[kHxSum][4];
@@ -135,28 +142,28 @@ __device__ __forceinline__ void hx_tile(const SmHx& S, int ra, int rb, int lane,
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    // weights 256^(5 - d), d = 6 and 7 rounded to the last place
+    // weights 16 256^(5 - d), d = 6 and 7 rounded to the last place
     const long long hi = ((long long)__float2int_rn(acc[0][k]) << 16) +
                          ((long long)__float2int_rn(acc[1][k]) << 8) +
                          __float2int_rn(acc[2][k]);
     const long long lo = ((long long)__float2int_rn(acc[3][k]) << 16) +
                          ((long long)__float2int_rn(acc[4][k]) << 8) +
-                         (__float2int_rn(acc[5][k]) +
-                          ((__float2int_rn(acc[6][k]) +
-                            ((__float2int_rn(acc[7][k]) + 128) >> 8) + 128) >> 8));
-    out[k] = (hi << 24) + lo;
+                         __float2int_rn(acc[5][k]);
+    const int tail = __float2int_rn(acc[6][k]) + ((__float2int_rn(acc[7][k]) + 128) >> 8);
+    out[k] = (((hi << 24) + lo) << 4) + ((tail + 8) >> 4);
   }
 }
 
-// An integer of hx_tile as the sum it stands for, v 2^(56 + ea + eb - 2 * 1076):
-// one conversion, the power of two added to the exponent field.
+// An integer of hx_tile as the sum it stands for, v 2^(52 + ea + eb - 2 * 1076):
+// one conversion, the power of two added to the exponent field; NaN for a bad row.
 __device__ __forceinline__ double hx_value(long long v, int ea, int eb) {
-  const int e = ea + eb - 2096;
-  double d = double(v);  // 0 or 2^0 .. 2^60
+  const int e = ea + eb - 2100;
+  double d = double(v);  // 0 or 2^0 .. 2^62
   if (abs(e) < 900) {
     const int hi = __double2hiint(d);
     return v == 0 ? d : __hiloint2double(hi + (e << 20), __double2loint(d));
   }
+  if (max(ea, eb) >= kHxBad) return __longlong_as_double(0x7ff8000000000000ll);
   const int e1 = max(-1022, min(1023, e)), e2 = max(-1022, min(1023, e - e1));
   return d * __longlong_as_double((long long)(e1 + 1023) << 52) *
          __longlong_as_double((long long)(e2 + 1023) << 52);
@@ -201,8 +208,8 @@ __global__ void __launch_bounds__(kHxThreads, 2)
     const int k = tid - 32;
     S.xv[k / 3][k % 3] = L.x[(size_t)3 * (ixe[k / 3] - 1) + k % 3];
   }
-  if (tid >= 64 && tid < 68) S.em[tid - 64] = 1;
-  if (tid == 68) S.fail = S.bad = 0;
+  if (tid >= 64 && tid < 64 + kHxRows) S.em[tid - 64] = 1;
+  if (tid == 255) S.fail = 0;
   // rows 68..71 are read with the row tiles around them
   for (int k = tid; k < kHxDig * 4 * 32; k += kHxThreads) {
     const int s = k >> 7, r = (k >> 5) & 3, c = k & 31;
@@ -283,30 +290,30 @@ __global__ void __launch_bounds__(kHxThreads, 2)
     const double sw = S.sw[gq];
     np[0] = tab(kTabH8 + part * 2) * sw;
     np[1] = tab(kTabH8 + part * 2 + 1) * sw;
-    int em[4] = {1, 1, 1, max(hx_exp(np[0]), hx_exp(np[1]))};
+    auto row_of = [part](int k, int j) {
+      return k < 5 ? 3 * (part * 5 + k) + j : 72 + 8 * j + part * 2 + k - 5;
+    };
+    // lane 3 k + j keeps the warp's largest exponent of row (k, j), lanes 21 and 22 of Np
+    int mine = 0;
 #pragma unroll
-    for (int k = 0; k < 7; ++k)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) em[j] = max(em[j], hx_exp(v[k][j]));
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      em[j] = __reduce_max_sync(0xffffffffu, em[j]);
-      if (lane == j) atomicMax(&S.em[j], em[j]);
+    for (int k = 0; k < 23; ++k) {
+      const int e = __reduce_max_sync(0xffffffffu, hx_exp(k < 21 ? v[k / 3][k % 3] : np[k - 21]));
+      mine = lane == k ? e : mine;
     }
+    if (lane < 23)
+      atomicMax(&S.em[lane < 21 ? row_of(lane / 3, lane % 3) : 60 + part * 2 + lane - 21],
+                mine == 0x7ff ? kHxBad : mine);
     __syncthreads();
+    // (all read before the first digit is stored: the compiler keeps their order)
+    int em[23];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) em[j] = S.em[j];
-    // a value that is not finite makes the element's entries NaN
-    if (tid == 0 && max(max(em[0], em[1]), max(em[2], em[3])) == 0x7ff) S.bad = 1;
+    for (int k = 0; k < 23; ++k)
+      em[k] = S.em[k < 21 ? row_of(k / 3, k % 3) : 60 + part * 2 + k - 21];
 #pragma unroll
-    for (int k = 0; k < 7; ++k)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const int row = k < 5 ? 3 * (part * 5 + k) + j : 72 + 8 * j + part * 2 + k - 5;
-        hx_digits(v[k][j], em[j], &S.dig[0][row][gq]);
-      }
-    hx_digits(np[0], em[3], &S.dig[0][60 + part * 2][gq]);
-    hx_digits(np[1], em[3], &S.dig[0][60 + part * 2 + 1][gq]);
+    for (int k = 0; k < 23; ++k) {
+      const int row = k < 21 ? row_of(k / 3, k % 3) : 60 + part * 2 + k - 21;
+      hx_digits(k < 21 ? v[k / 3][k % 3] : np[k - 21], em[k], &S.dig[0][row][gq]);
+    }
   }
   __syncthreads();
   // ---- the products -------------------------------------------------------------
@@ -333,19 +340,18 @@ __global__ void __launch_bounds__(kHxThreads, 2)
   __syncthreads();  // the digits are read: their space takes the sums
   {
     auto& R = S.r;
-    auto kind = [](int row) { return row < 60 ? row % 3 : row < 72 ? 3 : (row - 72) >> 3; };
-    const bool bad = S.bad != 0;
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
       const int t = wid + 8 * q;
       if (t >= kTiles) continue;
       int ra, rb;
       where(t, ra, rb);
+      const int er[2] = {S.em[ra + (lane >> 2)], S.em[ra + (lane >> 2) + 8]};
+      const int ec[2] = {S.em[rb + 2 * (lane & 3)], S.em[rb + 2 * (lane & 3) + 1]};
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int row = ra + (lane >> 2) + 8 * (k >> 1), col = rb + 2 * (lane & 3) + (k & 1);
-        const double d = bad ? __longlong_as_double(0x7ff8000000000000ll)
-                             : hx_value(res[q][k], S.em[kind(row)], S.em[kind(col)]);
+        const double d = hx_value(res[q][k], er[k >> 1], ec[k & 1]);
         if (t < 24) {
           if (col < 68) R.P[row][col] = d;
         } else if (t == 24) {
