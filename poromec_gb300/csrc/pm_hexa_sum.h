@@ -12,16 +12,19 @@
 // for problems in complex geometries", J. Comput. Phys. 37, 1980) takes 3,600, and
 // only the gradients, not the functions, are mapped at a point.  The FP64 pipe is
 // still what bounds them on many elements (79 % busy), the chain of sweeps on few.
-// Less rounding too: fields enter as differences, and one mid-side term is smaller
-// than its node's value (error of isw 2's forces on a smooth field 0.7e-16 of the
-// largest against 2.3e-16 with the functions).
+// Less rounding too: fields and coordinates enter as differences in every direction,
+// and one mid-side term is smaller than its node's value.  Errors against extended
+// precision, rms by output, with the functions and now: isw 2's forces 2.7e-16 and
+// 2.0e-16 on the 4^3 cube, 7.4e-16 and 2.6e-16 on the 18^3, the adjoint's gradients in
+// log E 1.9e-16 and 2.3e-16, 5.2e-16 and 2.8e-16, in log k 3.3e-16 and 2.5e-16, 6.2e-16
+// and 2.8e-16; jittered 8^3: forces 3.5e-16 and 2.6e-16, log E 2.8e-16 and 2.7e-16.
 //
 // One element per CTA of 192 threads: thread (point, direction) at the points,
 // one output per thread in each sweep; FP64 instructions are spread over the four
 // schedulers, since a warp's occupies one for 64 clocks.  Measured, before (every
 // function mapped, 64 threads) and now: isw 2's forces of the 40^3 cube 8.74 and
-// 2.91 ms, isw 4's 9.27 and 3.11, of the 2 x 2 x 40 column 0.43 and 0.03, 0.59 and
-// 0.05 (colours overlapped); the adjoint's two passes of the 32^3 cube 7.75 and 3.12.
+// 2.83 ms, isw 4's 9.27 and 2.96, of the 2 x 2 x 40 column 0.43 and 0.03, 0.59 and
+// 0.05 (colours overlapped); the adjoint's two passes of the 32^3 cube 7.75 and 3.01.
 constexpr int kSfThreads = 192;
 
 // index in the 3 x 3 x 3 grid (r + 3 s + 9 t) of each node, and the corners' in
@@ -42,13 +45,16 @@ template <SfOp OP>
 struct SmSf {
   static constexpr bool GRAD = OP == kSfGrad, BODY = OP == kSfRhs4;
   static constexpr int NC = GRAD ? 6 : 3;  // vector components: u, or lam and u_n
-  // linear fields: x, y, z, then the pressures the pass needs
-  static constexpr int NL = 3 + (GRAD ? 3 : OP == kSfRhs4 ? 2 : 1);
+  // linear fields: x, y, z, then the pressures the pass needs: the gradients of the
+  // first NG are taken, the values of NVF
+  static constexpr int NL = 3 + (GRAD ? 3 : OP == kSfRhs4 ? 2 : 1), NG = GRAD ? 5 : 4,
+                       NVF = GRAD ? 2 : OP == kSfApply ? 0 : 1;
   double C[NC][27];          // coefficients, then the sums
   double A[2][NC][36];      // [value, derivative][c][zy x]
   double B[NC][3][48];      // [c][r, s, t][z yx]
   double lin[NL][8];
-  double LB[NL][48];        // d/dr (z, y), d/ds (z, x), value (z, yx)
+  double LB[NG][32];        // d/dr (z, y), d/ds (z, x), d/dt (y, x)
+  double LV[NVF > 0 ? NVF : 1][32];  // value (z, yx)
   double JI[3][3][64];      // [x_j][xi_a]: dx_j / dxi_a, then det dxi_a / dx_j
   double rd[64], wq[64], w[64];  // 1 / det, the weight, weight times det
   double G[NC][3][64];      // physical gradients, then the natural fluxes
@@ -281,20 +287,32 @@ __global__ void __launch_bounds__(kSfThreads, 5)
   }
   if (tid >= 32 && tid < 32 + 12 * NC) sf_edge(S.C[(tid - 32) / 12], (tid - 32) % 12);
   // ---- linear fields, two directions --------------------------------------------
-  for (int k = tid; k < NL * 48; k += kSfThreads) {  // (one kind per warp, or nearly)
-    const int kind = k < NL * 8 ? 0 : k < NL * 16 ? 1 : 2;
-    const int f = kind == 2 ? (k - NL * 16) >> 5 : (k - kind * NL * 8) >> 3;
-    const int o = kind == 2 ? k - NL * 16 - 32 * f : k - kind * NL * 8 - 8 * f;
-    const double* c = S.lin[f] + 4 * (kind == 2 ? o >> 4 : o >> 2);
-    const double* wx = S.Lw[o & 3];
-    if (kind == 0) {  // d/dr at (z, y)
-      S.LB[f][o] = 0.5 * ((c[1] - c[0]) * wx[0] + (c[3] - c[2]) * wx[1]);
-    } else if (kind == 1) {  // d/ds at (z, x)
-      S.LB[f][8 + o] = 0.5 * ((c[2] - c[0]) * wx[0] + (c[3] - c[1]) * wx[1]);
-    } else {  // value at (z, y, x)
-      const double* wy = S.Lw[(o >> 2) & 3];
-      S.LB[f][16 + o] =
-          (c[0] * wx[0] + c[1] * wx[1]) * wy[0] + (c[2] * wx[0] + c[3] * wx[1]) * wy[1];
+  // (every derivative from the differences of the corners, then interpolated: what is
+  // rounded is the field's variation, not the field)
+  constexpr int NG = Sm::NG;
+  for (int k = tid; k < 32 * (NG + Sm::NVF); k += kSfThreads) {  // (nearly one kind per warp)
+    if (k < 16 * NG) {
+      const bool dr = k < 8 * NG;
+      const int m = dr ? k : k - 8 * NG, f = m >> 3, o = m & 7;
+      const double* c = S.lin[f] + 4 * (o >> 2);
+      const double* wx = S.Lw[o & 3];
+      if (dr)  // d/dr at (z, y)
+        S.LB[f][o] = 0.5 * ((c[1] - c[0]) * wx[0] + (c[3] - c[2]) * wx[1]);
+      else  // d/ds at (z, x)
+        S.LB[f][8 + o] = 0.5 * ((c[2] - c[0]) * wx[0] + (c[3] - c[1]) * wx[1]);
+    } else {
+      const int m = k - 16 * NG, o = m & 15;
+      const double *wx = S.Lw[o & 3], *wy = S.Lw[o >> 2];
+      if (m < 16 * NG) {  // d/dt at (y, x)
+        const double* c = S.lin[m >> 4];
+        S.LB[m >> 4][16 + o] = 0.5 * (((c[4] - c[0]) * wx[0] + (c[5] - c[1]) * wx[1]) * wy[0] +
+                                      ((c[6] - c[2]) * wx[0] + (c[7] - c[3]) * wx[1]) * wy[1]);
+      } else {  // value at (z, y, x): of the last field, the pass with two also of the first
+        const int z = ((m - 16 * NG) >> 4) & 1, v = (m - 16 * NG) >> 5;
+        const double* c = S.lin[Sm::NVF == 2 && v == 0 ? 3 : NL - 1] + 4 * z;
+        S.LV[v][16 * z + o] =
+            (c[0] * wx[0] + c[1] * wx[1]) * wy[0] + (c[2] * wx[0] + c[3] * wx[1]) * wy[1];
+      }
     }
   }
   __syncthreads();
@@ -312,9 +330,9 @@ __global__ void __launch_bounds__(kSfThreads, 5)
     const double* b = S.LB[f];
     n[0] = b[yx >> 2] * l0 + b[4 + (yx >> 2)] * l1;
     n[1] = b[8 + (yx & 3)] * l0 + b[12 + (yx & 3)] * l1;
-    n[2] = 0.5 * (b[32 + yx] - b[16 + yx]);
+    n[2] = b[16 + yx];
   };
-  auto value_lin = [&](int f) { return S.LB[f][16 + yx] * l0 + S.LB[f][32 + yx] * l1; };
+  auto value_lin = [&](int v) { return S.LV[v][yx] * l0 + S.LV[v][16 + yx] * l1; };
   {
     double n[3];
     grad_lin(j, n);
@@ -423,7 +441,7 @@ __global__ void __launch_bounds__(kSfThreads, 5)
     const double shl = S.G[j][j1][g] + S.G[j1][j][g];
     const double shu = S.G[3 + j][j1][g] + S.G[3 + j1][j][g];
     double v[3] = {-wq * rd * (S.G[j][j][g] * s + mc.c * mc.a * (shl * shu)), gk,
-                   j == 0 ? -S.w[g] * mc.imod_biot * value_lin(3) * value_lin(5) : 0.0};
+                   j == 0 ? -S.w[g] * mc.imod_biot * value_lin(0) * value_lin(1) : 0.0};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       double x = v[k];
@@ -446,11 +464,11 @@ __global__ void __launch_bounds__(kSfThreads, 5)
       const double e0 = S.G[j][j][g], e1 = S.G[j1][j1][g], e2 = S.G[j2][j2][g];
       double sn = (e0 + mc.b * e1 + mc.b * e2) * mc.a;
       if constexpr (OP == kSfResidual) {
-        const double pg = value_lin(3);
+        const double pg = value_lin(0);
         sn -= mc.coef_biot * pg;
         if (j == 0) S.S0[g] = S.w[g] * (mc.coef_biot * (e0 + e1 + e2) + mc.imod_biot * pg);
       } else if constexpr (OP == kSfRhs4) {
-        sn -= mc.coef_biot * value_lin(4);
+        sn -= mc.coef_biot * value_lin(0);
         if (j == 0) S.body[g] = S.w[g] * mc.pm_d;
       } else if (j == 0) {
         S.S0[g] = S.w[g] * mc.coef_biot * (e0 + e1 + e2);
