@@ -1517,10 +1517,18 @@ cudaError_t spmv(const PanelView& P, const double* val64, const double* x, doubl
   // small mesh launches only the CTAs it fills, and its fused dot sums that
   // many partials
   const int grid = std::max(1, std::min(kRedBlocks, (P.nact + 31) / 32));
-  // columns per trip (spmv_rows); with few nodes the compiler's loops: the product
-  // of the 3^3 cube takes 7.4 us with them, 7.7 to 8.1 with 4 or 5 (10^3: 14.4 and
-  // 15.3; 16^3, 18,785 nodes, 30.8 and 31.3; tetra 14^3, 24,389 nodes, 23.2 and 20.5)
-  const bool many = P.nact >= 24000;
+  // columns per trip (spmv_rows); with few nodes the compiler's loops: there the
+  // launch is a few trips of a warp, and the explicit ones gain nothing.  Microseconds,
+  // the compiler's loops and these, for the plain product, an iteration of PCG and one
+  // of MINRES: cube 3^3 7.4 and 7.7, -, -; tetra 8^3 (4,705 nodes) 14.5 and 14.5, 23.8
+  // and 24.6, 28.2 and 28.9; cube 12^3 (7,969) 18.6 and 18.6, 29.1 and 29.3, 33.4 and
+  // 34.2; tetra 10^3 (8,941) 16.6 and 16.5, 27.7 and 27.5, 32.6 and 31.9; column of 300
+  // layers (9,021) 17.9 and 16.5, 28.8 and 27.6, 33.5 and 32.3; tetra 13^3 (19,150)
+  // 20.7 and 18.6, 34.5 and 33.0, 40.7 and 39.1; cube 16^3 (18,241) 30.9 and 28.9, 43.2
+  // and 42.2, 52.9 and 50.7; tetra 20^3 55.7 and 45.7, 80.8 and 69.9, 95.3 and 84.5.
+  // Some larger cubes lose in the plain product (44^3 440 and 456, 50^3 638 and 655),
+  // the others gain 3 to 6 % (48^3 563 and 534).
+  const bool many = P.nact >= 8500;
   auto run = [&](auto few, auto most) {
     (many ? most : few)<<<grid, 256, 0, s>>>(P, val64, x, y, ks, partial, counter, nullptr);
   };
