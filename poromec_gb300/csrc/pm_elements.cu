@@ -161,14 +161,14 @@ __device__ __forceinline__ void sf_tetra10_v(T r, T s, T t, T* h) {
 
 // Shared geometry of one element: per integration point the weight
 // w = w_q det, the physical quadratic derivatives g[node][3], the linear
-// functions and their physical derivatives.
+// functions and (tetra10) their physical derivatives.
 template <bool HEXA, typename T>
 struct Geo {
   static constexpr int NEN = ET<HEXA>::NEN, NV = ET<HEXA>::NV, NGP = ET<HEXA>::NGP;
   T w[NGP];
   T g[NGP][NEN][3];
   T hp[NGP][NV];
-  T gp[NGP][NV][3];
+  T gp[HEXA ? 1 : NGP][NV][3];  // tetra10 only
   T xv[NV][3];
 };
 
@@ -210,8 +210,8 @@ template <typename T>
 __device__ bool point_geometry_tetra(Geo<false, T>& G, int gq, T r, T s, T t, T wq, T* huv);
 
 // The hexa's point geometry from the shape tables: the Jacobian from the
-// vertices, its inverse by one reciprocal of the determinant, and the
-// physical derivatives, with the table rows streamed from L1.
+// vertices, its inverse by one reciprocal of the determinant, and the quadratic
+// functions' physical derivatives, with the table rows streamed from L1.
 template <typename T>
 __device__ bool point_geometry_hexa_tab(Geo<true, T>& G, int gq) {
   constexpr int NEN = 20, NV = 8;
@@ -248,13 +248,7 @@ __device__ bool point_geometry_hexa_tab(Geo<true, T>& G, int gq) {
   const int lz = gq >> 4, ly = (gq >> 2) & 3, lx = gq & 3;
   G.w[gq] = T(cWG4[lx] * cWG4[ly] * cWG4[lz]) * det;
 #pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    const T hr = tab(kTabH8 + 8 + k), hs = tab(kTabH8 + 16 + k), ht = tab(kTabH8 + 24 + k);
-    G.hp[gq][k] = tab(kTabH8 + k);
-    G.gp[gq][k][0] = Ji[0][0] * hr + Ji[0][1] * hs + Ji[0][2] * ht;
-    G.gp[gq][k][1] = Ji[1][0] * hr + Ji[1][1] * hs + Ji[1][2] * ht;
-    G.gp[gq][k][2] = Ji[2][0] * hr + Ji[2][1] * hs + Ji[2][2] * ht;
-  }
+  for (int k = 0; k < NV; ++k) G.hp[gq][k] = tab(kTabH8 + k);
 #pragma unroll 4
   for (int k = 0; k < NEN; ++k) {
     const T ur = tab(kTabH20D + k), us = tab(kTabH20D + 20 + k), ut = tab(kTabH20D + 40 + k);
@@ -985,7 +979,7 @@ __global__ void __launch_bounds__(ET<false>::NT)
 
 // ---------------------------------------------------------------------------
 // Adjoint of the time-stepped solve.  Each step solves K du = F - A s - g0
-// with s = (u, dp) the previous state, where (from k_rhs4 and k_residual)
+// with s = (u, dp) the previous state, where (isw 4 and isw 2's forces)
 //   A s = [Kuu u_u + Kup dp ; Kpp_perm u_p],   g0 = [-body ; G_k],
 //   Kpp_perm = -dt perm int(grad N grad N),  G_k = dt perm rho_f int(grad N . g),
 // and then s += (du, du_p).  Every block is linear in one element parameter:
