@@ -5,67 +5,10 @@ import numpy as np
 import pytest
 
 import poromec_gb300 as pg
+from hexa_blocks import matrix
 from poromec_gb300 import meshgen
 
 pytestmark = pytest.mark.gpu
-
-# quadrature digits as the reference types them (Elmlib.f:3780-3962)
-_X4 = (-.861136311594053, -.339981043584856, .339981043584856, .861136311594053)
-_W4 = (.347854845137454, .652145154862546, .652145154862546, .347854845137454)
-_NODE = np.array([(1, 1, 1), (-1, 1, 1), (-1, -1, 1), (1, -1, 1), (1, 1, -1), (-1, 1, -1),
-                  (-1, -1, -1), (1, -1, -1), (0, 1, 1), (-1, 0, 1), (0, -1, 1), (1, 0, 1),
-                  (0, 1, -1), (-1, 0, -1), (0, -1, -1), (1, 0, -1), (1, 1, 0), (-1, 1, 0),
-                  (-1, -1, 0), (1, -1, 0)])
-
-
-def _matrix(X, e, grav, dt, T):
-    """K_e (60 displacements node by node, 8 pressures) in arithmetic T."""
-    x, w = np.array(_X4, T), np.array(_W4, T)
-    pts = np.array([(x[i], x[j], x[k]) for k in range(4) for j in range(4) for i in range(4)], T)
-    W = np.array([w[i] * w[j] * w[k] for k in range(4) for j in range(4) for i in range(4)], T)
-    hp, dl, dq = np.zeros((64, 8), T), np.zeros((64, 8, 3), T), np.zeros((64, 20, 3), T)
-    for k, c in enumerate(_NODE.astype(T)):
-        f, q = 1 + pts * c, 1 - pts * pts
-        for d in range(3):
-            a, b = (d + 1) % 3, (d + 2) % 3
-            if k < 8:
-                hp[:, k] = f[:, 0] * f[:, 1] * f[:, 2] / 8
-                dl[:, k, d] = c[d] * f[:, a] * f[:, b] / 8
-                dq[:, k, d] = c[d] * f[:, a] * f[:, b] * (
-                    pts[:, 0] * c[0] + pts[:, 1] * c[1] + pts[:, 2] * c[2] - 1 +
-                    pts[:, d] * c[d]) / 8
-            else:
-                g = np.where(c == 0, q, f)
-                dq[:, k, d] = (-2 * pts[:, d] if c[d] == 0 else c[d]) * g[:, a] * g[:, b] / 4
-    J = np.einsum("gki,kj->gij", dl, X.astype(T))
-    co = np.zeros_like(J)  # cofactors: co[a][j] of dx_j / dr_a
-    for a in range(3):
-        for j in range(3):
-            p, q, s, t = (a + 1) % 3, (a + 2) % 3, (j + 1) % 3, (j + 2) % 3
-            co[:, a, j] = J[:, p, s] * J[:, q, t] - J[:, p, t] * J[:, q, s]
-    det = (J[:, 0] * co[:, 0]).sum(1)
-    inv = co / det[:, None, None]
-    W = W * det
-    gp, gq = np.einsum("gaj,gka->gkj", inv, dl), np.einsum("gaj,gka->gkj", inv, dq)
-    E, nu = T(e[0]), T(e[1])
-    a, b = E * (1 - nu) / ((1 + nu) * (1 - 2 * nu)), nu / (1 - nu)
-    c = T(0.5) * (1 - 2 * nu) / (1 - nu)
-    fd = T(e[6]) * T(1e-6)
-    perm = T(e[2]) / (fd * np.sqrt((grav.astype(T) ** 2).sum()))
-    P = np.einsum("gik,gjl->ikjl", W[:, None, None] * gq, gq)
-    tr = np.einsum("ikjk->ij", P)
-    K = np.zeros((68, 68), T)
-    Kuu = np.zeros((20, 3, 20, 3), T)
-    for k in range(3):
-        for m in range(3):
-            Kuu[:, k, :, m] = (a * (P[:, k, :, k] + c * (tr - P[:, k, :, k])) if k == m else
-                               a * (b * P[:, k, :, m] + c * P[:, m, :, k]))
-    Kpu = -T(e[4]) * np.einsum("gl,gjk->ljk", W[:, None] * hp, gq).reshape(8, 60)
-    K[:60, :60], K[60:, :60], K[:60, 60:] = Kuu.reshape(60, 60), Kpu, Kpu.T
-    K[60:, 60:] = -(np.einsum("gl,gm->lm", W[:, None] * hp, hp) / T(e[3]) +
-                    T(dt) * perm * np.einsum("glk,gmk->lm", W[:, None, None] * gp, gp))
-    return K
-
 
 def _gpu_matrix(pb):
     m = pg.from_problem(pb)
@@ -108,10 +51,10 @@ def test_as_accurate_as_fp64_sums(taper, tilt):
     nd = np.asarray(pb["ix"])[0, :8] - 1
     args = (np.asarray(pb["x"])[nd], np.atleast_2d(pb["e"])[0], np.asarray(pb["gravity"], float),
             float(pb["dt"]))
-    exact = _matrix(*args, np.longdouble)
+    exact = matrix(*args, np.longdouble)
     d = np.sqrt(np.abs(np.diag(exact)))
     err = [np.asarray((K - exact) / np.outer(d, d), float) for K in
-           (_gpu_matrix(pb), _matrix(*args, np.float64))]
+           (_gpu_matrix(pb), matrix(*args, np.float64))]
     rms = [np.sqrt(np.mean(e * e)) for e in err]
     big = [np.abs(e).max() for e in err]
     print("taper %g tilt %g: rms %.2e (FP64 sums %.2e), largest %.2e (%.2e)"
