@@ -24,8 +24,8 @@
 // reductions and the scalar recurrences run in one warp, the quotients come from
 // a reciprocal by Newton's iteration, formed ahead where the divisor is known, and
 // a correction, and the results are broadcast.  The scalars stay in shared memory: in
-// registers they cost every thread some 20.  The panels are read through L1, which
-// holds them from one iteration to the next where they fit.
+// registers they cost every thread some 20.  The panels come from L2 in every
+// iteration (L1 hits 3 to 14 % of the sectors, L2 84 to 96 %).
 //
 // The recurrences and tests are those of the kernels in pm_sparse.cu
 // (k_pcg_update, k_sqmr_r, k_sqmr_x; Iters.f:299-595 and 6100-6439).  Every

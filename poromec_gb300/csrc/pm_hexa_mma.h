@@ -30,9 +30,10 @@
 // 16 x 8 over 8 warps, then a node pair per thread), two elements per SM.
 // Measured (assembly with the fused product, 40^3 cube, 64,000 elements): 10.2 ms
 // against 28.0 ms with DFMA sums (64 threads per element); a launch of 20
-// elements (2 x 2 x 40 column) 32 us against 184 us.  FP64 pipe 46 % busy: the
+// elements (2 x 2 x 40 column) 32 us against 184 us.  FP64 pipe 48 % busy: the
 // geometry, the blocks and the panel adds; the rest is the phases' latency with
-// two elements per SM (97 KB of digits each).
+// two elements per SM: 97 KB of digits each, and 128 registers a thread, either of
+// which alone keeps a third out.
 constexpr int kHxThreads = 256;
 constexpr int kHxRows = 96;     // 0..59 u, 60..67 Np, 68..71 zero, 72 + 8 k + l grad Np
 constexpr int kHxStride = 72;   // halves per digit row of 64 points: no bank conflicts
