@@ -28,7 +28,7 @@
 //
 // Per element: 256 threads (geometry: 4 threads per point, then 28 tiles of
 // 16 x 8 over 8 warps, then a node pair per thread), two elements per SM.
-// Measured (assembly with the fused product, 40^3 cube, 64,000 elements): 10.2 ms
+// Measured (assembly with the fused product, 40^3 cube, 64,000 elements): 10.1 ms
 // against 28.0 ms with DFMA sums (64 threads per element); a launch of 20
 // elements (2 x 2 x 40 column) 32 us against 184 us.  FP64 pipe 48 % busy: the
 // geometry, the blocks and the panel adds; the rest is the phases' latency with
@@ -321,6 +321,7 @@ __global__ void __launch_bounds__(kHxThreads, 2)
   // tiles 0..23: (16 I, 8 J), J >= 2 I, J <= 8; 24: Np 4..7; 25..27: grad Np
   constexpr int kTiles = 28, kPer = (kTiles + 7) / 8;
   long long res[kPer][4];
+  int er[kPer][2], ec[kPer][2];  // their rows' and columns' exponents
   auto where = [](int t, int& ra, int& rb) {
     if (t < 9) { ra = 0; rb = 8 * t; }
     else if (t < 16) { ra = 16; rb = 8 * (t - 7); }
@@ -336,6 +337,11 @@ __global__ void __launch_bounds__(kHxThreads, 2)
       int ra, rb;
       where(t, ra, rb);
       hx_tile(S, ra, rb, lane, res[q]);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        er[q][k] = S.em[ra + (lane >> 2) + 8 * k];
+        ec[q][k] = S.em[rb + 2 * (lane & 3) + k];
+      }
     }
   }
   __syncthreads();  // the digits are read: their space takes the sums
@@ -347,12 +353,10 @@ __global__ void __launch_bounds__(kHxThreads, 2)
       if (t >= kTiles) continue;
       int ra, rb;
       where(t, ra, rb);
-      const int er[2] = {S.em[ra + (lane >> 2)], S.em[ra + (lane >> 2) + 8]};
-      const int ec[2] = {S.em[rb + 2 * (lane & 3)], S.em[rb + 2 * (lane & 3) + 1]};
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int row = ra + (lane >> 2) + 8 * (k >> 1), col = rb + 2 * (lane & 3) + (k & 1);
-        const double d = hx_value(res[q][k], er[k >> 1], ec[k & 1]);
+        const double d = hx_value(res[q][k], er[q][k >> 1], ec[q][k & 1]);
         if (t < 24) {
           if (col < 68) R.P[row][col] = d;
         } else if (t == 24) {
